@@ -31,18 +31,17 @@
 // (a rotation of the same shuffle when D = 0).
 //
 // Steps run in chunks of 4, and rows always start on a chunk boundary, so
-// once per chunk a lane: reads one word of target codes (a sliding window,
-// prefetched two chunks ahead), exchanges 4 delay-line entries with one
-// 16-byte shared-memory access, stores one 32-bit traceback word (4 bits per
-// cell: low half's 4 steps in bits 15..0, high half's in bits 31..16, the
-// chunk's first step in the top nibble), and checks the chunk's maxima for
-// the best cell (the first maximum in row-then-slot order is recovered from
-// the chunk's 4 kept H values when the maximum grows).
+// once per chunk a lane: reads one word of target codes from a shared ring,
+// reads 4 delay-line entries with one 16-byte shared-memory access, stores
+// one 32-bit traceback word (4 bits per cell), and checks the chunk's maxima
+// for the best cell (the first maximum in row-then-slot order is recovered
+// from the chunk's 4 kept H values when the maximum grows).
 //
 // Long pairs with wide bands run in the cooperative form below: the warps of
 // one CTA share a pair strip by strip.
 
 #include <algorithm>
+#include <type_traits>
 
 #include "sw_common.cuh"
 
@@ -91,99 +90,66 @@ __device__ __forceinline__ unsigned tsel(int u) {
 }
 
 // ---------------------------------------------------------------------------
-// Pieces shared by the one-warp and the cooperative (several warps per pair)
-// kernels.
+// The pipeline of one warp, shared by the one-warp and the cooperative
+// (several warps per pair) kernels.
 // ---------------------------------------------------------------------------
+
+// The step's constants in registers: the compiler otherwise loads them from
+// the parameter bank (or rebuilds them) in every chunk.
+struct R16 {
+    unsigned ONE, NEG1, C7;  // 1, -1, 0x7fff7fff
+    unsigned MATCH2, MX, GO2, NGE2, Z2, NEG2;
+    __device__ __forceinline__ explicit R16(const K16& K)
+        : ONE(K.ONE), NEG1(K.NEG1), C7(0x7FFF7FFFu), MATCH2(K.MATCH2), MX(K.MX), GO2(K.GO2), NGE2(K.NGE2), Z2(K.Z2),
+          NEG2(K.NEG2) {
+        asm volatile("" : "+r"(ONE), "+r"(NEG1), "+r"(C7), "+r"(MATCH2), "+r"(MX), "+r"(GO2), "+r"(NGE2), "+r"(Z2),
+                     "+r"(NEG2));
+    }
+};
+
+// A value the compiler keeps in its register instead of rebuilding it.
+__device__ __forceinline__ void keep(int& x) { asm volatile("" : "+r"(x)); }
+__device__ __forceinline__ void keep(unsigned& x) { asm volatile("" : "+r"(x)); }
+
+// Shared memory by 32-bit address.
+__device__ __forceinline__ unsigned get_shared(unsigned addr) {
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void get_shared4(unsigned (&v)[4], unsigned addr) {
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void put_shared(unsigned addr, unsigned v, int pred) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\n@p st.shared.u32 [%0], %1;\n}" ::"r"(addr), "r"(v),
+                 "r"(pred) : "memory");
+}
+
+__device__ __forceinline__ void put_global(uint32_t* p, unsigned v, int pred) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\n@p st.global.u32 [%0], %1;\n}" ::"l"(
+                     __cvta_generic_to_global(p)),
+                 "r"(v), "r"(pred) : "memory");
+}
 
 // Per-lane DP state carried from step to step.
 struct Cells16 {
     unsigned hv, fv, hd, ml, el;  // H / F of the row above (this and the previous slot), M / E on the left
-    unsigned ma, mb;              // 32768 + slot - band_lo, 32768 + band_hi - slot per half (bit 15 set: in)
     unsigned qp;                  // query codes of the two rows (0x100 = never matches)
-    unsigned acc;                 // traceback nibbles of the chunk
+    unsigned acc;                 // traceback word of the chunk
 };
-
-__device__ __forceinline__ void cells_init(Cells16& c, const K16& K) {
-    c.hv = K.Z2;
-    c.fv = K.NEG2;
-    c.hd = K.Z2;
-    c.ml = K.NEG2;
-    c.el = K.NEG2;
-    c.ma = pack16(2768, 2768);  // out of band until the lane's first row starts
-    c.mb = pack16(20000, 20000);
-    c.qp = 0x01000100u;
-    c.acc = 0u;
-}
-
-// Target codes as 32-bit words of the whole target buffer, indexed from its
-// first aligned word; a chunk's 4 codes are a funnel shift of two words, and
-// the window slides one word per chunk with a load two chunks ahead.  Words
-// outside the buffer are clamped: they only ever feed out-of-band cells.
-struct TWin {
-    const uint32_t* w32;
-    int nwords;
-    long long pair_t;  // byte offset of the pair's codes from w32
-    unsigned w0, w1, w2;
-    int wi, tsh;
-    __device__ void setup(const SwArgs& a, const PairGeo& G, bool active) {
-        const long long tbase = (long long)(uintptr_t)a.t & ~3ll;
-        const long long t_total = active ? a.t_off[a.n_pairs] : 1;
-        const long long nw64 = (((long long)(uintptr_t)a.t + t_total - 1 - tbase) >> 2) + 1;
-        nwords = nw64 > 0x7fffffffll ? 0x7fffffff : (int)nw64;
-        w32 = reinterpret_cast<const uint32_t*>((uintptr_t)tbase);
-        pair_t = (long long)(uintptr_t)G.t - tbase;
-        w0 = w1 = w2 = 0u;
-        wi = 0;
-        tsh = 0;
-    }
-    // a negative index wraps to a large unsigned one and reads the last word
-    __device__ unsigned ld(int i) const { return __ldg(w32 + min((unsigned)i, (unsigned)(nwords - 1))); }
-    __device__ void start(int code_index, bool active) {  // window at code index `code_index` of the pair
-        const long long off = pair_t + (long long)code_index;
-        tsh = (int)(off & 3) * 8;
-        wi = (int)(off >> 2);
-        if (active) {
-            w0 = ld(wi);
-            w1 = ld(wi + 1);
-            w2 = ld(wi + 2);
-        }
-    }
-    __device__ unsigned window() const { return __funnelshift_r(w0, w1, tsh); }
-    __device__ void advance(bool active) {
-        w0 = w1;
-        w1 = w2;
-        ++wi;
-        if (active) w2 = ld(wi + 2);
-    }
-};
-
-// New rows for both halves of a lane: query codes and band intervals (the
-// high half's interval is expressed in the low half's slot, two steps later).
-__device__ __forceinline__ void row_start16(Cells16& c, int row, int j0, int qlen, int tlen, int W,
-                                            const int8_t* q) {
-    const int cq0 = row <= qlen ? (int)q[row - 1] : -1;
-    const int cq1 = row + 1 <= qlen ? (int)q[row] : -1;
-    c.qp = pack16((cq0 >= 0 && cq0 != 5) ? cq0 : 0x100, (cq1 >= 0 && cq1 != 5) ? cq1 : 0x100);
-    // interval bounds clamped into int16: an empty interval stays empty
-    const int lo0 = imin(imax(0, 1 - j0), 32000);
-    const int hi0 = row <= qlen ? imax(imin(W - 1, tlen - j0), -1) : -1;
-    const int lo1 = imin(imax(2, 2 - j0), 32000);
-    const int hi1 = row + 1 <= qlen ? imax(imin(W + 1, tlen - j0 + 1), -1) : -1;
-    c.ma = pack16(32768 - 1 - lo0, 32768 - 1 - lo1);
-    c.mb = pack16(32768 + hi0 + 1, 32768 + hi1 + 1);
-}
 
 // Four pipeline steps of one lane.  The first lane of the group takes its
-// row-above inputs from rv[] when `from_rv` (delay line or previous warp),
-// every other lane from lane k-1 by one shuffle of the packed (H.hi, F.hi).
-// MASKED: reset out-of-band cells (H = 0, M = E = F = -inf) at every step;
-// the caller drops it for chunks in which every lane of the warp stays
-// inside its band on all four steps (there the reset changes nothing) and
-// advances the band counters itself.
+// row-above inputs from rv[] (delay line or previous warp; `k0` is 0 there
+// and rv[] is 0 in every other lane), the others from lane k-1 by one shuffle
+// of the packed (H.hi, F.hi); lanes with `put` also store theirs at out_at.
+// MASKED: half words of m[] that are 0 mark
+// cells outside the band, which are reset (H = 0, M = E = F = -inf); the
+// caller drops it for chunks in which no lane of the warp is at a band edge.
 template <int L, bool TB, int EM, bool MASKED>
-__device__ __forceinline__ void chunk16(Cells16& c, const K16& K, const Grp<L>& grp, int src, unsigned tw,
-                                        unsigned tpv, bool from_rv, const unsigned (&rv)[4],
-                                        unsigned (&hk)[4], unsigned (&pko)[4]) {
+__device__ __forceinline__ void chunk16(Cells16& c, const K16& K, const R16& R, const Grp<L>& grp, int src,
+                                        unsigned tw, unsigned tpv, unsigned k0, const unsigned (&rv)[4],
+                                        const unsigned (&m)[4], unsigned (&hk)[4], unsigned out_at, int put) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
         // Every operand half is a biased value >= pmax and every difference
@@ -195,25 +161,30 @@ __device__ __forceinline__ void chunk16(Cells16& c, const K16& K, const Grp<L>& 
         // which runs at half rate and bounds the step.
         const unsigned tp = prmt(tw, tpv, tsel(u));
         const unsigned mis = flag2(c.qp ^ tp);  // 0: match, 1: mismatch
-        const unsigned diag = __vadd2(c.hd, K.MATCH2) - mis * K.MX;  // one multiply-add, no borrow
-        const unsigned fa = __vsub2(c.hv, K.GO2);
-        unsigned F = __viaddmax_u16x2(c.fv, K.NGE2, fa);  // max(F above - ext, H above - open)
-        unsigned M = __vimax3_u16x2(diag, F, K.Z2);
-        const unsigned ea = __vsub2(c.ml, K.GO2);
-        unsigned E = __viaddmax_u16x2(c.el, K.NGE2, ea);
-        unsigned H = umax2(M, E);
+        const unsigned diag = __vadd2(c.hd, R.MATCH2) - mis * R.MX;  // one multiply-add, no borrow
+        const unsigned fa = __vsub2(c.hv, R.GO2);
+        unsigned F = __viaddmax_u16x2(c.fv, R.NGE2, fa);  // max(F above - ext, H above - open)
+        unsigned M = __vimax3_u16x2(diag, F, R.Z2);
+        const unsigned ea = __vsub2(c.ml, R.GO2);
+        unsigned E = __viaddmax_u16x2(c.el, R.NGE2, ea);
+        if (MASKED) {
+            F = (F & m[u]) | (R.NEG2 & ~m[u]);
+            M = (M & m[u]) | (R.NEG2 & ~m[u]);
+            E = (E & m[u]) | (R.NEG2 & ~m[u]);
+        }
+        const unsigned H = MASKED ? __vimax3_u16x2(M, E, R.Z2) : umax2(M, E);  // in band H >= 0 anyway
         if (TB) {
             // Each flag is bit 15 of a half of (ordered difference + 0x7fff):
             // set when the difference is at least 1.  The classifier keeps
             // every difference within 15 bits, so the sums neither carry nor
             // borrow across halves (the 32-bit x + 0x7fff7fff may carry, and
             // the subtraction that follows takes the carry back).
-            const unsigned hb = H * K.ONE + 0x7FFF7FFFu;
-            const unsigned n1 = diag * K.NEG1 + hb;                        // H != diag
-            const unsigned n2 = F * K.NEG1 + hb;                           // H != F
-            const unsigned fc = fa * K.NEG1 + (F * K.ONE + 0x7FFF7FFFu);   // F extends (F above - ext > H above - open)
-            unsigned ec = 0u;                                              // E extends
-            if (EM == 0) ec = ea * K.NEG1 + (E * K.ONE + 0x7FFF7FFFu);     //   open > ext: E_left - ext > M_left - open
+            const unsigned hb = H * R.ONE + R.C7;
+            const unsigned n1 = diag * R.NEG1 + hb;                // H != diag
+            const unsigned n2 = F * R.NEG1 + hb;                   // H != F
+            const unsigned fc = fa * R.NEG1 + (F * R.ONE + R.C7);  // F extends (F above - ext > H above - open)
+            unsigned ec = 0u;                                      // E extends
+            if (EM == 0) ec = ea * R.NEG1 + (E * R.ONE + R.C7);    //   open > ext: E_left - ext > M_left - open
             if (EM == 2) ec = c.el - E + K.EB2;          //   open < ext: E == E_left - ext (ties extend)
             // sign-replicated high bytes: [n1.lo n1.hi n2.lo n2.hi], [fc.lo fc.hi ec.lo ec.hi]
             const unsigned w1 = prmt(n1, n2, 0xFDB9u);
@@ -221,97 +192,42 @@ __device__ __forceinline__ void chunk16(Cells16& c, const K16& K, const Grp<L>& 
             const unsigned b = (w1 & (0x01010101u << u)) | (w2 & (0x10101010u << u));
             c.acc = u == 0 ? b : (c.acc | b);
         }
-        if (MASKED) {
-            // in-band mask: slot - lo >= 0 and hi - slot >= 0 per half, kept as
-            // counters biased by 32768 (they never leave [0, 65535], so plain
-            // adds suffice); bit 15 of both set = in band
-            c.ma = __vadd2(c.ma, ONE2);
-            c.mb = __vsub2(c.mb, ONE2);
-            const unsigned m = prmt(c.ma & c.mb, 0u, 0xBB99u);  // 0xFFFF per in-band half
-            H = (H & m) | (K.Z2 & ~m);
-            F = (F & m) | (K.NEG2 & ~m);
-            M = (M & m) | (K.NEG2 & ~m);
-            E = (E & m) | (K.NEG2 & ~m);
-        }
         const unsigned pk = prmt(H, F, 0x7632u);  // (H.hi, F.hi)
-        unsigned sh = grp.shfl(pk, src);
-        if (from_rv) sh = rv[u];
+        put_shared(out_at + 4 * u, pk, put);
+        const unsigned sh = grp.shfl(pk, src) * k0 + rv[u];
         c.hd = c.hv;
         c.hv = prmt(sh, H, 0x5410u);  // low: row above (lane k-1 high), high: own low
         c.fv = prmt(sh, F, 0x5432u);
         c.ml = M;
         c.el = E;
         hk[u] = H;
-        pko[u] = pk;
     }
 }
 
-// True when every cell of the lane's next chunk (4 steps, both halves) is in
-// band: the first step's lower-bound counters and the last step's upper-
-// bound counters both have bit 15 set.
-__device__ __forceinline__ bool chunk_in_band(const Cells16& c) {
-    return ((c.ma + ONE2) & (c.mb - 4u * ONE2) & 0x80008000u) == 0x80008000u;
-}
-
-// A chunk with or without the band reset: the unmasked form when the whole
-// warp stays in band (warp-uniform decision).
-template <int L, bool TB, int EM>
-__device__ __forceinline__ void chunk16_any(Cells16& c, const K16& K, const Grp<L>& grp, int src, unsigned tw,
-                                            unsigned tpv, bool from_rv, const unsigned (&rv)[4],
-                                            unsigned (&hk)[4], unsigned (&pko)[4]) {
-    if (__all_sync(FULL_MASK, chunk_in_band(c))) {
-        chunk16<L, TB, EM, false>(c, K, grp, src, tw, tpv, from_rv, rv, hk, pko);
-        c.ma = __vadd2(c.ma, 4u * ONE2);
-        c.mb = __vsub2(c.mb, 4u * ONE2);
-    } else {
-        chunk16<L, TB, EM, true>(c, K, grp, src, tw, tpv, from_rv, rv, hk, pko);
-    }
-}
-
-// Best-cell bookkeeping of a chunk: `lb` is the running maximum per half (the
-// row maximum under x-drop); when it grows, the first of the chunk's 4 steps
-// that reaches it gives the position (global step, or slot under x-drop).
-template <bool XD>
-__device__ __forceinline__ void best16(unsigned& lb, int& pos0, int& pos1, const unsigned (&hk)[4], int gstep,
-                                       int d) {
-    const unsigned nb = __vimax3_u16x2(lb, __vimax3_u16x2(hk[0], hk[1], hk[2]), hk[3]);
-    if (nb != lb) {
-        // per half, the steps before the first that reaches nb, counted for
-        // both halves at once: nb >= hk[u] in each half, so the plain
-        // subtractions do not borrow across halves, and flag2 is 1 while
-        // hk[u] < nb
-        const unsigned e0 = flag2(nb - hk[0]);
-        const unsigned e01 = e0 & flag2(nb - hk[1]);
-        const unsigned e012 = e01 & flag2(nb - hk[2]);
-        const unsigned u = e0 + e01 + e012;  // 0..3 in each half
-        const unsigned inc = nb ^ lb;
-        if (inc & 0xFFFFu) pos0 = (XD ? d : gstep) + (int)(u & 0xFFFFu);
-        if (inc >> 16) pos1 = (XD ? d - 2 : gstep) + (int)(u >> 16);
-        lb = nb;
-    }
-}
-
-// Best-cell bookkeeping without x-drop, branch-free: when a half's running
-// maximum grows, that half's 4 H values of the chunk and the chunk's first
-// global step are kept (a per-half select); the first step that reaches the
-// final maximum is found once, after the DP, from the kept values.  The
-// maximum only grows on a strictly larger value, so the kept chunk is the
-// one in which the final maximum first appears.
+// Best-cell bookkeeping, branch-free: when a half's running maximum grows,
+// that half's 4 H values of the chunk and the chunk's first step are kept (a
+// per-half select); the first step that reaches the final maximum is found
+// once, from the kept values.  The maximum only grows on a strictly larger
+// value, so the kept chunk is the one in which the final maximum first
+// appears.
 struct BestTrack16 {
+    unsigned lb;  // running maximum per half
     unsigned sv[4];
     int g_lo, g_hi;
     __device__ __forceinline__ void init(unsigned z2) {
-        sv[0] = sv[1] = sv[2] = sv[3] = z2;
+        lb = sv[0] = sv[1] = sv[2] = sv[3] = z2;
         g_lo = g_hi = 0;
     }
-    // Run by the whole warp (every caller's chunk loop is warp-uniform): the
-    // selects are skipped in the chunks where no lane's maximum grows.
-    __device__ __forceinline__ void update(unsigned& lb, const unsigned (&hk)[4], int g0) {
+    // Run by the whole warp.  VOTE: the selects are skipped in the chunks
+    // where no lane's maximum grows (with row maxima, reset at every row,
+    // some lane's always does).
+    template <bool VOTE>
+    __device__ __forceinline__ void update(const unsigned (&hk)[4], int g0, unsigned c7) {
         const unsigned nb = __vimax3_u16x2(lb, __vimax3_u16x2(hk[0], hk[1], hk[2]), hk[3]);
-        if (__any_sync(FULL_MASK, nb != lb)) {
+        if (!VOTE || __any_sync(FULL_MASK, nb != lb)) {
             // nb >= lb in each half and the difference stays within 15 bits:
-            // bit 15 of difference + 0x7fff is "grew", spread over the half
-            const unsigned up = prmt(nb - lb + 0x7FFF7FFFu, 0u, 0xBB99u);
+            // bit 15 of difference + 0x7fff (c7) is "grew", spread over the half
+            const unsigned up = prmt(nb - lb + c7, 0u, 0xBB99u);
 #pragma unroll
             for (int u = 0; u < 4; ++u) sv[u] = (hk[u] & up) | (sv[u] & ~up);
             g_lo = (up & 1u) ? g0 : g_lo;
@@ -319,8 +235,8 @@ struct BestTrack16 {
             lb = nb;
         }
     }
-    // Global steps of the first cell of each half that holds its maximum.
-    __device__ __forceinline__ void positions(unsigned lb, int& pos0, int& pos1) const {
+    // Steps of the first cell of each half that holds its maximum.
+    __device__ __forceinline__ void positions(int& pos0, int& pos1) const {
         int u0 = 3, u1 = 3;
 #pragma unroll
         for (int u = 2; u >= 0; --u) {
@@ -332,24 +248,413 @@ struct BestTrack16 {
     }
 };
 
-// Best cell of a lane (non-x-drop): the first maximum of each half, from its
-// global step, as (score, row, slot).
-template <int L>
-__device__ __forceinline__ void lane_best16(unsigned lb, int pos0, int pos1, unsigned Z, int g, int k, int P,
-                                            int& bh, int& bi, int& bd) {
+// (score, row, slot) ordering of the best cell: higher score, then earlier
+// row, then earlier slot.
+__device__ __forceinline__ bool better_cell(int oh, int oi, int od, int bh, int bi, int bd) {
+    return oh > bh || (oh == bh && (oi < bi || (oi == bi && od < bd)));
+}
+
+// Progress flags between the warps of a CTA: the writer publishes with a
+// release store after its ring store, the reader polls with acquire loads;
+// neither waits for the thread's outstanding global loads or stores (a block
+// fence would).
+__device__ __forceinline__ int ld_acquire_cta(const int* p) {
+    int v;
+    asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v)
+                 : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_cta(int* p, int v, int pred) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\n@p st.release.cta.shared.b32 [%0], %1;\n}" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(p)),
+                 "r"(v), "r"(pred) : "memory");
+}
+
+// Shared memory of one lane group: the delay line (or, cooperative, this
+// warp's output ring), two copies of a ring of target codes, the band masks.
+struct GroupSmem {
+    uint32_t* ring;
+    unsigned char* codes;
+    uint4* tab;
+};
+__host__ __device__ inline size_t group_smem_bytes(int ring, int tring, int tabn) {
+    return (size_t)ring * 4 + 2 * (size_t)tring + ((size_t)tabn + 2) * 16;
+}
+__device__ __forceinline__ GroupSmem group_smem(const SwArgs& a, unsigned char* base, int group) {
+    GroupSmem s;
+    unsigned char* p = base + (size_t)group * group_smem_bytes(a.ring, a.tring, a.tabn);
+    s.ring = reinterpret_cast<uint32_t*>(p);
+    s.codes = p + (size_t)a.ring * 4;
+    s.tab = reinterpret_cast<uint4*>(s.codes + 2 * (size_t)a.tring);
+    return s;
+}
+
+// What the cooperating warps of a CTA share (NW > 1).
+struct CoopLinks {
+    const uint32_t* ring_in;   // the previous warp's output ring
+    int* prog;                 // per warp: ring entries published
+    int* cons;                 // per warp: entries of the previous warp no longer needed
+};
+
+// Runs the strips w, w + NW, ... of one pair (NW = 1: all of them) and leaves
+// the traceback words, the best cell per half (non-x-drop) or the row maxima
+// (x-drop).
+//
+// What bounds it is the instruction count of a 4-step chunk, and with few
+// pairs on the GPU the latency of its dependent steps, so everything that is
+// not a cell is kept off the chunk:
+//  * Target codes come from a shared ring of the codes around the band,
+//    refilled 2L codes at a time (loaded one refill ahead).  Chunk starts of
+//    a strip lie at multiples of 4 codes from the strip's first, except that
+//    odd lanes are off by 2, so two copies of the ring (the second shifted by
+//    2 codes) make every chunk one aligned word load.
+//  * Codes outside the target read 0xFF, which matches nothing.  Cells left
+//    of the target then compute H = 0 and E, F < 0 by themselves (E, F = 0
+//    with a free gap open), which gives every cell inside the target the
+//    values, and every decision a walk can take, of cells that read 0 and
+//    -inf there; cells right of the target or below the query feed no cell
+//    inside, and their values come from cells inside by penalties only, so
+//    they never pass the best cell's score, and a cell that equals it lies in
+//    a later row (or a later slot of the row).  So only the band's own edges
+//    (slots < 0 and >= W) need a reset, and these are the same chunks of
+//    every row: the masks of a chunk are one 16-byte load from a table.
+//    With 32 lanes, chunks in which no lane starts or ends a row run without
+//    masks, and the table holds only the chunks near a row's ends.  Row maxima (x-drop) must not see the cells right of the target:
+//    strips that reach its end add that bound to the masks.
+//  * Rows start on a counter (one compare a chunk); the next row's query
+//    codes are loaded one strip ahead by all lanes at once.
+// Measured on one B200 against the form that kept target words per lane in
+// registers, counted every row's band per step and polled every chunk:
+// instructions per 4-step chunk 190 from 284 (32 lanes, x-drop, W = 129: 180),
+// 204 from 260 (8 warps); steps of a lone warp 133 cycles from 226; GCUPS on
+// uniform pairs 711 from 617 (3,000 x 1,500, W = 181), 775 from 628 (888 x
+// 3,000, W = 601, 4 warps), 900 from 621 (444 x 2,000, W = 3,201, 8 warps),
+// 545 from 445 (20,000 x 150, W = 65, 16 lanes).
+// Registers: the step needs ~110 to keep its constants and both copies of the
+// chunk's values at hand.  Bounds of 95, 80 and 72 registers (20, 24 and 28
+// warps an SM instead of 16) ran the same pairs at 709, 656 and 551 GCUPS
+// (32 lanes) and a lone warp's steps 10, 31 and 35% slower, so the kernels ask
+// for 16 warps an SM.
+template <int L, int NW, bool TB, bool XD, int EM>
+__device__ __forceinline__ void sw16_rows(const SwArgs& a, const PairGeo& G, bool active, const Grp<L>& grp,
+                                          const GroupSmem& sm, int w, int nstrips, int n_chunks, int last_chunk,
+                                          uint32_t* bits, int2* rowmax, const CoopLinks& lk, BestTrack16& bt) {
+    constexpr int V = 2 * L, VS = V * NW;  // rows of a strip, rows between this warp's strips
+    constexpr bool COOP = NW > 1;
+    // The 8-warp class (wide bands) bounds each warp's lead over the warp that
+    // reads it as well: lane 31 waits until its reader has taken the entries
+    // it is about to overwrite, so a ring of a.ring entries (1024) serves
+    // periods up to COOP_PMAX instead of needing P + 8.  A warp's lag behind
+    // its predecessor then stays within [132, a.ring + 128] steps; the lags
+    // of the NW links sum to P, so with NW * 132 <= P <= NW * (a.ring + 128)
+    // the warps cannot all be waiting at once.
+    constexpr bool BP = NW == 8;
+    const K16& K = a.k16;
+    const int k = grp.k;
+    const int qlen = G.qlen, tlen = G.tlen, W = G.W, P = G.P;
+    const int nch = P >> 2, nE = (W - 1) >> 2;  // chunks of a period; chunk of a row's last slot (low half)
+    const int c0 = G.off - G.hb;                // j = row + c0 + slot
+    const int8_t* __restrict__ q = G.q;
+
+    // ---- target codes: ring byte r of copy A is code R0 + r, of copy B code R0 + r + 2 ----
+    const long long tbase = (long long)(uintptr_t)a.t & ~3ll;
+    const uint32_t* __restrict__ w32 = reinterpret_cast<const uint32_t*>((uintptr_t)tbase);
+    long long nw64 = 1;
+    if (active) nw64 = (((long long)(uintptr_t)a.t + a.t_off[a.n_pairs] - 1 - tbase) >> 2) + 1;
+    const unsigned last_word = nw64 > 0x7fffffffll ? 0x7ffffffeu : (unsigned)(nw64 - 1);
+    const long long pair_t = active ? (long long)(uintptr_t)G.t - tbase : 0ll;
+    int tmask = a.tring - 1;
+    keep(tmask);
+    const int R0 = V * w + c0;
+    auto raw_codes = [&](int idx, unsigned& lo, unsigned& hi) {  // the two aligned words over codes idx .. idx+3
+        if (active) {
+            const int wi = (int)((pair_t + (long long)idx) >> 2);  // a negative index reads the last word
+            lo = __ldg(w32 + min((unsigned)wi, last_word));
+            hi = __ldg(w32 + min((unsigned)(wi + 1), last_word));
+        }
+    };
+    auto put_codes = [&](int wd, int copy, int idx, unsigned lo, unsigned hi) {
+        unsigned v = __funnelshift_r(lo, hi, (int)((pair_t + (long long)idx) & 3) * 8);
+        const int below = idx < 0 ? imin(-idx, 4) : 0, above = idx + 4 > tlen ? imin(idx + 4 - tlen, 4) : 0;
+        if (below) v |= below == 4 ? 0xFFFFFFFFu : (1u << (8 * below)) - 1u;
+        if (above) v |= above == 4 ? 0xFFFFFFFFu : ~(0xFFFFFFFFu >> (8 * above));
+        *reinterpret_cast<uint32_t*>(sm.codes + copy * a.tring + ((4 * wd) & tmask)) = v;
+    };
+    for (int x = k; x < 2 * nch; x += L) {  // codes of the first period, both copies
+        const int wd = x >> 1, copy = x & 1, idx = R0 + 4 * wd + 2 * copy;
+        unsigned lo = 0u, hi = 0u;
+        raw_codes(idx, lo, hi);
+        put_codes(wd, copy, idx, lo, hi);
+    }
+    // refills: L words (2L codes of both copies) per event, one per lane
+    const int f_copy = k / (L / 2);
+    int f_wd = nch + k % (L / 2);
+    unsigned f_lo = 0u, f_hi = 0u;
+    raw_codes(R0 + 4 * f_wd + 2 * f_copy, f_lo, f_hi);
+    auto refill = [&]() {
+        put_codes(f_wd, f_copy, R0 + 4 * f_wd + 2 * f_copy, f_lo, f_hi);
+        f_wd += L / 2;
+        raw_codes(R0 + 4 * f_wd + 2 * f_copy, f_lo, f_hi);
+    };
+
+    // ---- band masks by chunk of the row (32 lanes: chunks 0..32, then the last 33) ----
+    const int n_tab = L == 32 ? imin(nch, MASK_ROWS) : nch;
+    for (int x = k; x < n_tab; x += L) {
+        const int cc = x <= 32 || L < 32 ? x : x + nch - n_tab;
+        unsigned mm[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int t = 4 * cc + u;
+            mm[u] = (t <= W - 1 ? 0xFFFFu : 0u) | (t >= 2 && t <= W + 1 ? 0xFFFF0000u : 0u);
+        }
+        sm.tab[x] = make_uint4(mm[0], mm[1], mm[2], mm[3]);
+    }
+    if (k == 0) {
+        const unsigned i = K.init_pk();
+        sm.tab[a.tabn] = make_uint4(0u, 0u, 0u, 0u);
+        sm.tab[a.tabn + 1] = make_uint4(i, i, i, i);
+    }
+    if (!COOP)
+        for (int x = k; x < a.ring; x += L) sm.ring[x] = K.init_pk();
+    __syncwarp();
+
+    // ---- per-lane state ----
+    Cells16 c;
+    c.hv = c.hd = K.Z2;
+    c.fv = c.ml = c.el = K.NEG2;
+    c.qp = 0x01000100u;
+    c.acc = 0u;
+    unsigned tpv = 0u;
+    bt.init(K.Z2);
+    // byte offset of the lane's chunk in the mask table (n_tab entries on, the
+    // next row starts; lane k's first row starts at chunk k)
+    const int y_end = 16 * n_tab;
+    int y = y_end - 16 * k;
+    const unsigned codes_at = (unsigned)__cvta_generic_to_shared(sm.codes + (k & 1) * a.tring);
+    const unsigned tab_at = (unsigned)__cvta_generic_to_shared(sm.tab);
+    int pos = P - VS - 2 * k - 2 * (k & 1);  // ring byte of the chunk's codes
+    int tbi = COOP ? (w - (NW - 1)) * nch * L + k : k;          // word of the chunk's traceback bits
+    unsigned tb_lim = COOP ? 0u : (unsigned)(last_chunk + 1) * L;  // no words before a lane's first row
+    const unsigned tb_all = (unsigned)(last_chunk + 1) * L;
+    const int src = (k + L - 1) & (L - 1);
+    const int D = P - 4 * L;  // delay-line steps, a multiple of 4 (0: a rotation of the shuffle)
+    const bool from_rv = k == 0 && (COOP || D > 0);
+    const int to_ring = k == L - 1 && (COOP ? !a.coop_stall : D > 0) ? 1 : 0;
+    const unsigned k0 = from_rv ? 0u : 1u;
+    int rmask = a.ring - 1;
+    keep(rmask);
+    const unsigned ring_at = (unsigned)__cvta_generic_to_shared(sm.ring);
+    // The first lane reads its entries from the ring (row 0 above the first
+    // strip and strips past the query: a constant entry), the others zeros.
+    const unsigned const_at = (unsigned)__cvta_generic_to_shared(sm.tab + a.tabn) + (from_rv ? 16u : 0u);
+    const unsigned src_at = COOP ? (unsigned)__cvta_generic_to_shared(lk.ring_in) : ring_at;
+    unsigned in_at = COOP || !from_rv ? const_at : src_at;
+    unsigned in_step = COOP || !from_rv ? 0u : 4u;
+    int jump = VS - P;
+    keep(jump);
+    const R16 R(K);
+    // Cooperative waits: the last progress read from the previous / next warp,
+    // and how far ahead of its need a warp that has to wait lets its
+    // predecessor run, so that it polls once per several chunks.  The lags of
+    // the NW links sum to P, so a wait for a lag of 132 + ahead <= P / NW
+    // cannot close the ring.
+    int seen = 0, freed = 0;
+    const int ahead = COOP ? imin(64, (P / NW - 132) & ~3) : 0;
+    const int w_prev = (w + NW - 1) % NW;
+    const int prev_end = COOP && w_prev < nstrips ? (((nstrips - 1 - w_prev) / NW + 1) * P + 4 * L + 4) & ~3 : 0;
+
+    int row = V * (w - NW) + 2 * k + 1;  // the lane's low row of the current period
+    unsigned nqp = 0x01000100u, nmb = 0u;
+    int rq0 = row + VS <= qlen ? (int)q[row + VS - 1] : -1;
+    int rq1 = row + VS + 1 <= qlen ? (int)q[row + VS] : -1;
+    unsigned mb = 0u;  // x-drop: 32768 + slots inside the target per half, from the row's start
+    // x-drop: the finished row's maximum, written by all lanes at once in the next period
+    BestTrack16 fin;
+    if (XD) fin.init(K.Z2);
+    auto write_rows = [&](const BestTrack16& b, int kk) {
+        const int r = V * (w + NW * kk) + 2 * k + 1;
+        int p0, p1;
+        b.positions(p0, p1);
+        const int at = kk * P + 4 * k;
+        if (active && kk >= 0) {
+            if (r <= qlen) rowmax[r - 1] = make_int2((lo16(b.lb) - (int)K.Z) * K.G, p0 - at);
+            if (r + 1 <= qlen) rowmax[r] = make_int2((hi16(b.lb) - (int)K.Z) * K.G, p1 - at - 2);
+        }
+    };
+
+    // Polls a progress flag until it reaches `need`.  Bounded: after the
+    // limit, or once any wait in the grid gave up (every later wait then ends
+    // within ~1k spins), record and go on.
+    auto wait_for = [&](int& have, const int* flag, int need) {
+        int spins = 0;
+        // the smallest of the lanes' own reads: uniform, and no lane goes on before its own read allows it
+        while ((have = __reduce_min_sync(FULL_MASK, ld_acquire_cta(flag))) < need) {
+            if (++spins > a.coop_spin_limit ||
+                ((spins & 1023) == 0 &&
+                 __any_sync(FULL_MASK, (*(volatile int*)a.err & (int)GMF_SWF_TIMEOUT) != 0))) {
+                if (k == 0) atomicOr(a.err, (int)GMF_SWF_TIMEOUT);
+                break;
+            }
+            __nanosleep(40);
+        }
+    };
+
+    int kk = -1;             // the group's period (lane 0's strip)
+    int next_period = 0;     // chunk at which it ends
+    // Cooperative: everything that happens only every few chunks, behind one
+    // compare a chunk: NW refills of 64 codes a period, one every 33 chunks (a
+    // period has at least 33 * NW); waits; and, with back-pressure, the
+    // reader's progress every 8 chunks.
+    int limit = 0;  // chunk at which events() must run again
+    int next_fill = 0x7fffffff, fills = 0;
+    const int lag = 4 * L - (w == 0 ? P : 0);  // entry e = local step + lag of the previous warp
+    bool reading = false;
+    auto events = [&](int gc) {
+        if (gc >= next_fill) {
+            refill();
+            next_fill = --fills > 0 ? gc + 33 : 0x7fffffff;
+        }
+        limit = imin(next_fill, next_period);
+        if (reading) {
+            const int e = 4 * gc + lag;
+            if (seen < e + 4) wait_for(seen, lk.prog + w_prev, imin(e + 4 + ahead, prev_end));
+            limit = imin(limit, ((seen - lag - 4) >> 2) + 1);
+        }
+        if (BP) {
+            // the slots of steps t .. t+3 held steps t - ring .. t - ring + 3
+            if (freed < 4 * gc + 4 - a.ring) wait_for(freed, lk.cons + (w + 1) % NW, 4 * gc + 4 - a.ring);
+            limit = imin(limit, ((freed + a.ring - 4) >> 2) + 1);
+            // the previous warp's entries before this chunk's are no longer needed (also when this strip
+            // reads none)
+            st_release_cta(lk.cons + w, 4 * gc + lag, k == 0 ? 1 : 0);
+            limit = imin(limit, gc + 8);
+        }
+        limit = imax(limit, gc + 1);  // a wait that gave up
+    };
+    // One chunk.  MASKED: some lane may be at a band edge; SHIFT: bytes the
+    // lanes move on in the mask table (0 in the middle of the rows).
+    auto chunk = [&](int gc, auto masked_, auto shift_) {
+        constexpr bool MASKED = decltype(masked_)::value;
+        constexpr int SHIFT = decltype(shift_)::value;
+        if (SHIFT && gc == next_period) {  // lane 0 of the group starts a strip
+            next_period += nch;
+            ++kk;
+            row += VS;
+            if (COOP) {
+                next_fill = kk > 0 ? gc : 0x7fffffff;
+                fills = NW;
+                const int s0 = w + NW * kk;
+                reading = s0 >= 1 && s0 < nstrips;
+                if (from_rv) {
+                    in_at = reading ? src_at : const_at;
+                    in_step = reading ? 4u : 0u;
+                }
+                limit = gc;
+            } else if (kk > 0) {
+                refill();
+            }
+            nqp = pack16((rq0 >= 0 && rq0 != 5) ? rq0 : 0x100, (rq1 >= 0 && rq1 != 5) ? rq1 : 0x100);
+            if (XD) {
+                const int hi0 = row <= qlen ? imax(imin(W - 1, tlen - row - c0), -1) : -1;
+                const int hi1 = row + 1 <= qlen ? imax(imin(W + 1, tlen - row - c0 + 1), -1) : -1;
+                nmb = pack16(32768 + hi0 + 1, 32768 + hi1 + 1);
+                write_rows(fin, kk - 2);
+            }
+            rq0 = row + VS <= qlen ? (int)q[row + VS - 1] : -1;
+            rq1 = row + VS + 1 <= qlen ? (int)q[row + VS] : -1;
+        }
+        if (COOP && gc >= limit) events(gc);
+        unsigned rv[4];
+        get_shared4(rv, in_at + in_step * (unsigned)((4 * gc + (COOP ? lag : -D)) & rmask));
+        if (SHIFT && y == y_end) {  // the lane starts its next row (the high half two steps later)
+            y = 0;
+            c.qp = nqp;
+            pos += jump;
+            if (COOP) {
+                tbi += (NW - 1) * nch * L;
+                tb_lim = tb_all;
+            }
+            if (XD) {
+                mb = nmb;
+                fin = bt;
+                bt.lb = K.Z2;
+            }
+        }
+        const unsigned tw = get_shared(codes_at + (unsigned)(pos & tmask));
+        unsigned m[4] = {0u, 0u, 0u, 0u};
+        if (MASKED) {
+            get_shared4(m, tab_at + (unsigned)y);
+            if (XD) {  // the slots still inside the target against the step, as bit 15 per half
+#pragma unroll
+                for (int u = 0; u < 4; ++u) m[u] &= prmt(mb - (unsigned)(u + 1) * ONE2, 0u, 0xBB99u);
+            }
+        }
+        unsigned hk[4];
+        chunk16<L, TB, EM, MASKED>(c, K, R, grp, src, tw, tpv, k0, rv, m, hk,
+                                   ring_at + 4 * (unsigned)((4 * gc) & rmask), to_ring);
+        // published before the global store, so the release does not wait on it
+        if (COOP) st_release_cta(lk.prog + w, 4 * gc + 4, to_ring);
+        tpv = prmt(tw, tpv, 0x4344u);  // this chunk's last code, for the next chunk's high half
+        pos += 4;
+        y += SHIFT;
+        if (XD) mb -= 4u * ONE2;
+        if (TB) {
+            put_global(bits + tbi, c.acc, (L == 32 && !COOP) || (unsigned)tbi < tb_lim);
+            tbi += L;
+        }
+        bt.template update<!XD>(hk, 4 * gc, R.C7);
+        __syncwarp();
+    };
+    using True = std::true_type;
+    using False = std::false_type;
+    if (L < 32 || nE <= 32) {
+        for (int gc = 0; gc < n_chunks; ++gc) chunk(gc, True{}, std::integral_constant<int, 16>{});
+    } else {
+        // rows start in chunks 0..31 of a period and end from chunk nE on and, in the next period, up to chunk 31
+        const int y_jump = 16 * (nch > n_tab ? 34 - (nch - nE) : nE - 32);
+        int gc = 0;
+        for (int base = 0;; base += nch) {
+            const int e1 = imin(base + 32, n_chunks);
+            for (; gc < e1; ++gc) chunk(gc, True{}, std::integral_constant<int, 16>{});
+            if (gc >= n_chunks) break;
+            const int e2 = imin(base + nE, n_chunks);
+            // x-drop: rows that end right of the target keep the masks
+            if (XD && V * (w + NW * kk + 1) + c0 + W - 1 > tlen)
+                for (; gc < e2; ++gc) chunk(gc, True{}, std::integral_constant<int, 0>{});
+            else
+                for (; gc < e2; ++gc) chunk(gc, False{}, std::integral_constant<int, 0>{});
+            y += y_jump;
+        }
+    }
+    if (XD && n_chunks > 0) {
+        // rows not yet written: the last finished one of the lanes that started a strip in the last
+        // period, and the current one
+        const int my = n_chunks - 1 >= k ? (n_chunks - 1 - k) / nch : -1;
+        if (my == kk) write_rows(fin, kk - 1);
+        write_rows(bt, my);
+    }
+}
+
+// Best cell of a warp's lanes (non-x-drop): the first maximum of each half,
+// from its step in the warp's schedule, as (score, row, slot).
+template <int L, int NW>
+__device__ __forceinline__ void lane_best16(const BestTrack16& bt, unsigned Z, int g, int k, int P, int w, int& bh,
+                                            int& bi, int& bd) {
     constexpr int V = 2 * L;
-    const int v0 = (lo16(lb) - (int)Z) * g, v1 = (hi16(lb) - (int)Z) * g;  // true scores
+    int pos0, pos1;
+    bt.positions(pos0, pos1);
+    const int v0 = (lo16(bt.lb) - (int)Z) * g, v1 = (hi16(bt.lb) - (int)Z) * g;  // true scores
     int r0 = 0, s0 = 0, r1 = 0, s1 = 0;
     if (v0 > 0) {
         const int tt = pos0 - 2 * (2 * k);
         const int s = tt / P;
-        r0 = s * V + 2 * k + 1;
+        r0 = (w + NW * s) * V + 2 * k + 1;
         s0 = tt - s * P;
     }
     if (v1 > 0) {
         const int tt = pos1 - 2 * (2 * k + 1);
         const int s = tt / P;
-        r1 = s * V + 2 * k + 2;
+        r1 = (w + NW * s) * V + 2 * k + 2;
         s1 = tt - s * P;
     }
     bh = v0;
@@ -362,17 +667,28 @@ __device__ __forceinline__ void lane_best16(unsigned lb, int pos0, int pos1, uns
     }
 }
 
-// (score, row, slot) ordering of the best cell: higher score, then earlier
-// row, then earlier slot.
-__device__ __forceinline__ bool better_cell(int oh, int oi, int od, int bh, int bi, int bd) {
-    return oh > bh || (oh == bh && (oi < bi || (oi == bi && od < bd)));
+// The best cell of the lanes of a group, in every lane.
+template <int L>
+__device__ __forceinline__ void group_best16(const Grp<L>& grp, int& bh, int& bi, int& bd) {
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+        const int oh = grp.xr(bh, o);
+        const int oi = grp.xr(bi, o);
+        const int od = grp.xr(bd, o);
+        if (better_cell(oh, oi, od, bh, bi, bd)) {
+            bh = oh;
+            bi = oi;
+            bd = od;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
-// One group of L lanes per pair.
+// One group of L lanes per pair.  The traceback walk runs later, in
+// sw_walk_kernel.
 // ---------------------------------------------------------------------------
 template <int L, bool TB, bool XD, int EM>
-__device__ void sw16_group(const SwArgs& a, int p, const Grp<L>& grp, uint32_t* ring) {
+__device__ void sw16_group(const SwArgs& a, int p, const Grp<L>& grp, const GroupSmem& sm) {
     constexpr int V = 2 * L;
     PairGeo G = load_geo(a, p);
     const int k = grp.k;
@@ -380,12 +696,9 @@ __device__ void sw16_group(const SwArgs& a, int p, const Grp<L>& grp, uint32_t* 
     const bool bad = has && (G.hb < 0 || G.hb > a.max_hb);
     bool active = has && !bad && G.qlen > 0 && G.tlen > 0;
     if (has && !active && k == 0) write_empty<TB>(a, p, bad);
-    const int qlen = G.qlen, tlen = G.tlen, W = G.W;
-    const int P = sw16_period(W, L);
-    G.P = P;
-    const int D = P - 4 * L;  // delay-line steps, a multiple of 4
-    const bool use_ring = D > 0;
-    const int rmask = a.ring - 1;
+    if (bad) G.W = 1;
+    const int qlen = G.qlen, W = G.W;
+    G.P = sw16_period(W, L);
 
     const unsigned long long tbw = (TB && active) ? sw16_tb_words_l(qlen, W, L) : 0ull;
     uint32_t* ws = ws_alloc<L>(a, grp, tbw + (XD && active ? 2ull * qlen : 0ull), active && (TB || XD));
@@ -393,111 +706,14 @@ __device__ void sw16_group(const SwArgs& a, int p, const Grp<L>& grp, uint32_t* 
         if (k == 0) write_empty<TB>(a, p, true);
         active = false;
     }
-    uint32_t* bits = ws;
     int2* rowmax = (XD && active) ? reinterpret_cast<int2*>(ws + tbw) : nullptr;
     const int nstrips = (qlen + V - 1) / V;
-    const int my_last = active ? (nstrips - 1) * P + 2 * ((qlen - 1) % V) + W - 1 : -1;
-    const int loop_last = __reduce_max_sync(FULL_MASK, my_last);
+    const int my_last = active ? (nstrips - 1) * G.P + 2 * ((qlen - 1) % V) + W - 1 : -1;
     const int last_chunk = my_last >> 2;  // -1 when inactive
+    const int n_chunks = __reduce_max_sync(FULL_MASK, last_chunk) + 1;
 
-    const K16& K = a.k16;
-    for (int x = k; x < a.ring; x += L) ring[x] = K.init_pk();
-    __syncwarp();
-    TWin tw;
-    tw.setup(a, G, active);
-
-    const int8_t* __restrict__ q = G.q;
-    const int c0 = G.off - G.hb;  // j = row + c0 + d
-    int d = -4 * k;               // slot of the low half at the chunk start (x-drop bookkeeping)
-    int until = k;                // chunks until the lane's next row start (every P / 4 chunks)
-    int tbi = k;                  // word of the chunk's traceback bits: (g0 / 4) * L + k
-    const int tb_end = last_chunk * L + k;
-    int row = 2 * k + 1 - V;      // row of the low half (advanced by V at each row start)
-    Cells16 c;
-    cells_init(c, K);
-    unsigned tpv = 0u;
-    unsigned lb = K.Z2;  // best H so far per half (non-x-drop) / row max (x-drop)
-    int pos0 = 0, pos1 = 0;
     BestTrack16 bt;
-    bt.init(K.Z2);
-    unsigned rv[4] = {0u, 0u, 0u, 0u};  // delay-line entries of the chunk
-    const int src = (k + L - 1) & (L - 1);
-    const bool from_rv = use_ring && k == 0;
-    const int dW0 = (W - 1) & ~3, dW1 = (W + 1) & ~3;  // chunks that end a row (x-drop)
-
-    // The lane's next row (query codes, band counters, target window) is
-    // prepared by the whole group in the chunk where the group's lane 0
-    // starts its row (until == k there), and taken up k chunks later: the
-    // loads and bounds run once per period for all lanes instead of one lane
-    // at a time.
-    unsigned nqp = 0u, nma = 0u, nmb = 0u, nw0 = 0u, nw1 = 0u, nw2 = 0u;
-    int nwi = 0, ntsh = 0;
-
-    for (int g0 = 0; g0 <= loop_last; g0 += 4) {
-        if (until == k) {
-            Cells16 nx;
-            row_start16(nx, row + V, row + V + c0, qlen, tlen, W, q);
-            TWin tn = tw;
-            tn.start(row + V + c0 - 1, active);
-            nqp = nx.qp;
-            nma = nx.ma;
-            nmb = nx.mb;
-            nw0 = tn.w0;
-            nw1 = tn.w1;
-            nw2 = tn.w2;
-            nwi = tn.wi;
-            ntsh = tn.tsh;
-        }
-        if (until == 0) {  // both halves start new rows (the high half two steps later)
-            until = P >> 2;
-            row += V;
-            c.qp = nqp;
-            c.ma = nma;
-            c.mb = nmb;
-            tw.w0 = nw0;
-            tw.w1 = nw1;
-            tw.w2 = nw2;
-            tw.wi = nwi;
-            tw.tsh = ntsh;
-            tpv = 0u;
-            if (XD) {
-                lb = K.Z2;
-                pos0 = 0;
-                pos1 = 0;
-            }
-        }
-        if (from_rv) {
-            const uint4 r = *reinterpret_cast<const uint4*>(ring + ((g0 - D) & rmask));
-            rv[0] = r.x;
-            rv[1] = r.y;
-            rv[2] = r.z;
-            rv[3] = r.w;
-        }
-        const unsigned twin = tw.window();
-        unsigned hk[4], pk[4];
-        chunk16_any<L, TB, EM>(c, K, grp, src, twin, tpv, from_rv, rv, hk, pk);
-        // ---- once per chunk ----
-        tpv = prmt(twin, tpv, 0x4344u);  // this chunk's last code, for the next chunk's high half
-        tw.advance(active);
-        if (TB && tbi <= tb_end) bits[tbi] = c.acc;
-        tbi += L;
-        if (use_ring && k == L - 1)
-            *reinterpret_cast<uint4*>(ring + (g0 & rmask)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        if (XD)
-            best16<XD>(lb, pos0, pos1, hk, g0, d);
-        else
-            bt.update(lb, hk, g0);
-        if (XD) {
-            if (d == dW0 && row <= qlen && row >= 1) rowmax[row - 1] = make_int2((lo16(lb) - (int)K.Z) * K.G, pos0);
-            if (d == dW1 && row + 1 <= qlen && row >= 1) rowmax[row] = make_int2((hi16(lb) - (int)K.Z) * K.G, pos1);
-        }
-        __syncwarp();
-        --until;
-        if (XD) {
-            d += 4;
-            if (d == P) d = 0;
-        }
-    }
+    sw16_rows<L, 1, TB, XD, EM>(a, G, active, grp, sm, 0, nstrips, n_chunks, last_chunk, ws, rowmax, CoopLinks{}, bt);
     __syncwarp();
 
     int bh, bi, bd;
@@ -505,66 +721,42 @@ __device__ void sw16_group(const SwArgs& a, int p, const Grp<L>& grp, uint32_t* 
         if (active && k == 0) record_rowmax(a, p, rowmax);
         xdrop_best<L>(grp, rowmax, qlen, a.x_drop, active, bh, bi, bd);
     } else {
-        bt.positions(lb, pos0, pos1);
-        lane_best16<L>(lb, pos0, pos1, K.Z, K.G, k, P, bh, bi, bd);
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) {
-            const int oh = grp.xr(bh, o);
-            const int oi = grp.xr(bi, o);
-            const int od = grp.xr(bd, o);
-            if (better_cell(oh, oi, od, bh, bi, bd)) {
-                bh = oh;
-                bi = oi;
-                bd = od;
-            }
-        }
+        lane_best16<L, 1>(bt, a.k16.Z, a.k16.G, k, G.P, 0, bh, bi, bd);
+        group_best16<L>(grp, bh, bi, bd);
         if (!active) bh = 0;
     }
-    const int qe = bh > 0 ? bi : 0;
-    const int te = bh > 0 ? bi + G.off - G.hb + bd : 0;
     if (active && k == 0) {
         a.score[p] = bh;
-        a.q_end[p] = qe;
-        a.t_end[p] = te;
+        a.q_end[p] = bh > 0 ? bi : 0;
+        a.t_end[p] = bh > 0 ? bi + G.off - G.hb + bd : 0;
+        if (TB) record_walk(a, p, ws, L);
     }
-    if (!TB) return;
-    if (a.defer_walk) {  // the traceback walk runs later, in sw_walk_kernel
-        if (active && k == 0) record_walk(a, p, bits, L);
-        return;
-    }
-
-    RunWriter rw;
-    uint32_t* runs = ws_alloc<L>(a, grp, (unsigned long long)qe + te + 1, active && bh > 0);
-    const bool runs_ok = !(active && bh > 0) || runs != nullptr;
-    if (!runs_ok && k == 0) atomicOr(a.err, (int)GMF_SWF_WORKSPACE);
-    rw.init(runs);
-    Layout16<L> lay{bits, P, W, qlen};
-    int qs = 0, ts = 0;
-    walk<L>(grp, lay, G, a, qe, te, bh, active && runs_ok && bh > 0, rw, qs, ts);
-    finish_cigar<L>(a, grp, p, active, rw, runs_ok, qs, ts);
 }
 
+// Warps take pairs in the list's order (longest first).  The first pair of
+// each warp is fixed: pairs go to one warp of every block before a second
+// one, and to different schedulers of the SM in the blocks of later waves, so
+// a short list spreads over the SMs instead of filling the first blocks.
 template <int L, bool TB, bool XD, int EM>
-__global__ void __launch_bounds__(128) sw16_kernel(SwArgs a) {
-    extern __shared__ uint4 sw16_ring4[];
-    uint32_t* sw16_ring = reinterpret_cast<uint32_t*>(sw16_ring4);
+__global__ void __launch_bounds__(128, 4) sw16_kernel(SwArgs a) {
+    extern __shared__ uint4 sw16_smem[];
     constexpr int GPW = 32 / L;  // pairs per warp
     constexpr int CLS = L == 8 ? CLS_I16_L8 : (L == 16 ? CLS_I16_L16 : CLS_I16_L32);
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
+    const int wib = threadIdx.x >> 5, wpb = (int)blockDim.x >> 5;
     const int gi = lane / L;
-    uint32_t* ring = sw16_ring + ((size_t)wib * GPW + gi) * a.ring;
+    const GroupSmem sm = group_smem(a, reinterpret_cast<unsigned char*>(sw16_smem), wib * GPW + gi);
     Grp<L> grp(lane);
     const int count = a.queue[N_CLASSES + CLS];
     const int32_t* list = a.lists + (size_t)CLS * a.n_pairs;
-    for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&a.queue[CLS], GPW);
-        base = __shfl_sync(FULL_MASK, base, 0);
-        if (base >= count) break;
+    const int wave = (int)blockIdx.x / a.sms;
+    int base = (((wib + wpb - wave % wpb) % wpb) * (int)gridDim.x + (int)blockIdx.x) * GPW;
+    while (base < count) {
         const int idx = base + gi;
         const int p = idx < count ? list[idx] : -1;
-        sw16_group<L, TB, XD, EM>(a, p, grp, ring);
+        sw16_group<L, TB, XD, EM>(a, p, grp, sm);
+        if (lane == 0) base = atomicAdd(&a.queue[CLS], GPW) + (int)gridDim.x * wpb * GPW;
+        base = __shfl_sync(FULL_MASK, base, 0);
     }
 }
 
@@ -583,41 +775,17 @@ __global__ void __launch_bounds__(128) sw16_kernel(SwArgs a) {
 // entries ahead of its reader, so the 2- and 4-warp classes use rings of
 // R >= P + 8 entries and no back-pressure.  The 8-warp class (periods up to
 // COOP_PMAX) adds back-pressure instead and keeps 1,024-entry rings: its
-// writers also wait for their readers (see sw16_coop_pair).  Each writer
+// writers also wait for their readers (see sw16_rows).  Each writer
 // publishes its progress after every chunk (ring store, then a release store
 // of the flag); each reader polls the flag with acquire loads and an
 // iteration limit, after which it records GMF_SWF_TIMEOUT and goes on.
 // Traceback words land at the same (global step, lane) positions as in the
-// one-warp layout, so the walk (warp 0, after a block barrier) is unchanged.
+// one-warp layout, so the walk is unchanged.
 // ---------------------------------------------------------------------------
-
-// Progress flags between the warps of a CTA: the writer publishes with a
-// release store after its ring store, the reader polls with acquire loads;
-// neither waits for the thread's outstanding global loads or stores (a block
-// fence would).
-__device__ __forceinline__ int ld_acquire_cta(const int* p) {
-    int v;
-    asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v)
-                 : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_cta(int* p, int v) {
-    asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "r"(v)
-                 : "memory");
-}
-
 template <int NW, bool TB, bool XD, int EM>
-__device__ void sw16_coop_pair(const SwArgs& a, int p, uint32_t* rings, int* prog, int* cons, int (*sbest)[3],
+__device__ void sw16_coop_pair(const SwArgs& a, int p, unsigned char* smem, int* prog, int* cons, int (*sbest)[3],
                                uint32_t** sws) {
     constexpr int L = 32, V = 64;
-    // The 8-warp class (wide bands) bounds each warp's lead over the warp that
-    // reads it as well: lane 31 waits until its reader has taken the entries
-    // it is about to overwrite, so a ring of a.ring entries (1024) serves
-    // periods up to COOP_PMAX instead of needing P + 8.  A warp's lag behind
-    // its predecessor then stays within [132, a.ring + 128] steps; the lags
-    // of the NW links sum to P, so with NW * 132 <= P <= NW * (a.ring + 128)
-    // the warps cannot all be waiting at once.
-    constexpr bool BP = NW == 8;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     Grp<32> grp(lane);
     PairGeo G = load_geo(a, p);
@@ -626,9 +794,9 @@ __device__ void sw16_coop_pair(const SwArgs& a, int p, uint32_t* rings, int* pro
         if (threadIdx.x == 0) write_empty<TB>(a, p, bad);
         return;
     }
-    const int qlen = G.qlen, tlen = G.tlen, W = G.W;
-    const int P = sw16_period(W, L);
-    G.P = P;
+    const int qlen = G.qlen, W = G.W;
+    G.P = sw16_period(W, L);
+    const int P = G.P;
     const int nstrips = (qlen + V - 1) / V;
     const int my_last = (nstrips - 1) * P + 2 * ((qlen - 1) % V) + W - 1;  // global step of the last cell
     const int last_chunk = my_last >> 2;
@@ -648,168 +816,22 @@ __device__ void sw16_coop_pair(const SwArgs& a, int p, uint32_t* rings, int* pro
         if (threadIdx.x == 0) write_empty<TB>(a, p, true);
         return;
     }
-    uint32_t* bits = ws;
     int2* rowmax = XD ? reinterpret_cast<int2*>(ws + tbw) : nullptr;
 
-    const K16& K = a.k16;
-    TWin tw;
-    tw.setup(a, G, true);
-    const int8_t* __restrict__ q = G.q;
-    const int c0 = G.off - G.hb;
     const int kk_last = w < nstrips ? (nstrips - 1 - w) / NW : -1;  // this warp's last strip (local index)
-    const int loop_end = (kk_last + 1) * P + 4 * L + 4;             // drains what the next warp may read
-    uint32_t* ring_out = rings + (size_t)w * a.ring;
-    const int wprev = (w + NW - 1) % NW;
-    const uint32_t* ring_in = rings + (size_t)wprev * a.ring;
-    const int rmask = a.ring - 1;
-    const unsigned INIT = K.init_pk();
-
-    int d = -4 * lane;  // slot of the low half at the chunk start (x-drop bookkeeping)
-    int until = lane;   // chunks until the lane's next row start (every P / 4 chunks)
-    int tbi = 0x3fffffff;  // word of the chunk's traceback bits ((t + gofs) / 4 * L + lane), none before a row
-    const int tb_end = last_chunk * L + lane;
-    int kk = -1;        // local index of the lane's current strip
-    int row = 0, gofs = 0;
-    Cells16 c;
-    cells_init(c, K);
-    unsigned tpv = 0u, lb = K.Z2;
-    int pos0 = 0, pos1 = 0;
+    // drains what the next warp may read
+    const int n_chunks = kk_last >= 0 ? ((kk_last + 1) * P + 4 * L + 4) >> 2 : 0;
+    const GroupSmem sm = group_smem(a, smem, w);
+    const CoopLinks lk{group_smem(a, smem, (w + NW - 1) % NW).ring, prog, cons};
     BestTrack16 bt;
-    bt.init(K.Z2);
-    unsigned rv[4] = {INIT, INIT, INIT, INIT};
-    const int src = (lane + 31) & 31;
-    const int dW0 = (W - 1) & ~3, dW1 = (W + 1) & ~3;
-
-    // the lane's next row, prepared by the whole warp when lane 0 starts its
-    // strip (until == lane there) and taken up lane chunks later
-    unsigned nqp = 0u, nma = 0u, nmb = 0u, nw0 = 0u, nw1 = 0u, nw2 = 0u;
-    int nwi = 0, ntsh = 0;
-
-    if (kk_last >= 0) {
-        for (int t = 0; t < loop_end; t += 4) {
-            if (until == lane) {
-                const int nrow = (w + NW * (kk + 1)) * V + 2 * lane + 1;
-                Cells16 nx;
-                row_start16(nx, nrow, nrow + c0, qlen, tlen, W, q);
-                TWin tn = tw;
-                tn.start(nrow + c0 - 1, true);
-                nqp = nx.qp;
-                nma = nx.ma;
-                nmb = nx.mb;
-                nw0 = tn.w0;
-                nw1 = tn.w1;
-                nw2 = tn.w2;
-                nwi = tn.wi;
-                ntsh = tn.tsh;
-            }
-            if (until == 0) {
-                until = P >> 2;
-                ++kk;
-                const int s = w + NW * kk;
-                row = s * V + 2 * lane + 1;
-                gofs = (s - kk) * P;  // local step -> step of the one-warp schedule
-                tbi = ((t + gofs) >> 2) * L + lane;
-                c.qp = nqp;
-                c.ma = nma;
-                c.mb = nmb;
-                tw.w0 = nw0;
-                tw.w1 = nw1;
-                tw.w2 = nw2;
-                tw.wi = nwi;
-                tw.tsh = ntsh;
-                tpv = 0u;
-                if (XD) {
-                    lb = K.Z2;
-                    pos0 = 0;
-                    pos1 = 0;
-                }
-            }
-            if (lane == 0) {
-                const int s0 = w + NW * kk;  // lane 0 starts its strips at t = kk * P
-                if (s0 >= 1 && s0 < nstrips) {
-                    const int e = t + 4 * L - (w == 0 ? P : 0);
-                    int spins = 0;
-                    while (ld_acquire_cta(prog + wprev) < e + 4) {
-                        // bounded: after the limit, or once any wait in the grid gave up
-                        // (every later wait then ends within ~1k spins), record and go on
-                        if (++spins > a.coop_spin_limit ||
-                            ((spins & 1023) == 0 && (*(volatile int*)a.err & (int)GMF_SWF_TIMEOUT))) {
-                            atomicOr(a.err, (int)GMF_SWF_TIMEOUT);
-                            break;
-                        }
-                        __nanosleep(20);
-                    }
-                    const uint4 r = *reinterpret_cast<const uint4*>(ring_in + (e & rmask));
-                    rv[0] = r.x;
-                    rv[1] = r.y;
-                    rv[2] = r.z;
-                    rv[3] = r.w;
-                } else {
-                    rv[0] = rv[1] = rv[2] = rv[3] = INIT;  // row 0, or a strip past the query
-                }
-                // the previous warp's entries before t + 4 * L (+ 4), in its step
-                // numbering, are no longer needed (also when this strip reads none)
-                if (BP) st_release_cta(cons + w, t + 4 * L + 4 - (w == 0 ? P : 0));
-            }
-            const unsigned twin = tw.window();
-            unsigned hk[4], pk[4];
-            chunk16_any<32, TB, EM>(c, K, grp, src, twin, tpv, lane == 0, rv, hk, pk);
-            tpv = prmt(twin, tpv, 0x4344u);
-            tw.advance(true);
-            if (lane == 31) {  // publish before the global store, so the release does not wait on it
-                if (BP) {
-                    // the slots of steps t .. t+3 held steps t - ring .. t - ring + 3
-                    const int need = t + 4 - a.ring;
-                    int spins = 0;
-                    while (ld_acquire_cta(cons + (w + 1) % NW) < need) {
-                        if (++spins > a.coop_spin_limit ||
-                            ((spins & 1023) == 0 && (*(volatile int*)a.err & (int)GMF_SWF_TIMEOUT))) {
-                            atomicOr(a.err, (int)GMF_SWF_TIMEOUT);
-                            break;
-                        }
-                        __nanosleep(20);
-                    }
-                }
-                *reinterpret_cast<uint4*>(ring_out + (t & rmask)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                if (!a.coop_stall) st_release_cta(prog + w, t + 4);
-            }
-            const int g0 = t + gofs;
-            if (TB && tbi <= tb_end) bits[tbi] = c.acc;
-            tbi += L;
-            if (XD)
-                best16<XD>(lb, pos0, pos1, hk, g0, d);
-            else
-                bt.update(lb, hk, g0);
-            if (XD && kk >= 0) {
-                if (d == dW0 && row <= qlen) rowmax[row - 1] = make_int2((lo16(lb) - (int)K.Z) * K.G, pos0);
-                if (d == dW1 && row + 1 <= qlen) rowmax[row] = make_int2((hi16(lb) - (int)K.Z) * K.G, pos1);
-            }
-            __syncwarp();
-            --until;
-            if (XD) {
-                d += 4;
-                if (d == P) d = 0;
-            }
-        }
-    }
-    if (BP && lane == 0 && kk_last >= 0) st_release_cta(cons + w, 0x7fffffff);  // reads nothing more
+    sw16_rows<L, NW, TB, XD, EM>(a, G, true, grp, sm, w, nstrips, n_chunks, last_chunk, ws, rowmax, lk, bt);
+    if (NW == 8 && lane == 0 && kk_last >= 0) st_release_cta(cons + w, 0x7fffffff, 1);  // reads nothing more
     __syncthreads();  // every traceback word and row maximum is written
 
     int bh = 0, bi = 0, bd = 0;
     if (!XD) {
-        bt.positions(lb, pos0, pos1);
-        lane_best16<L>(lb, pos0, pos1, K.Z, K.G, lane, P, bh, bi, bd);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const int oh = grp.xr(bh, o);
-            const int oi = grp.xr(bi, o);
-            const int od = grp.xr(bd, o);
-            if (better_cell(oh, oi, od, bh, bi, bd)) {
-                bh = oh;
-                bi = oi;
-                bd = od;
-            }
-        }
+        lane_best16<L, NW>(bt, a.k16.Z, a.k16.G, lane, P, w, bh, bi, bd);
+        group_best16<L>(grp, bh, bi, bd);
         if (lane == 0) {
             sbest[w][0] = bh;
             sbest[w][1] = bi;
@@ -832,33 +854,17 @@ __device__ void sw16_coop_pair(const SwArgs& a, int p, uint32_t* rings, int* pro
                 bd = sbest[x][2];
             }
     }
-    const int qe = bh > 0 ? bi : 0;
-    const int te = bh > 0 ? bi + G.off - G.hb + bd : 0;
     if (lane == 0) {
         a.score[p] = bh;
-        a.q_end[p] = qe;
-        a.t_end[p] = te;
+        a.q_end[p] = bh > 0 ? bi : 0;
+        a.t_end[p] = bh > 0 ? bi + G.off - G.hb + bd : 0;
+        if (TB) record_walk(a, p, ws, L);
     }
-    if (!TB) return;
-    if (a.defer_walk) {  // the traceback walk runs later, in sw_walk_kernel
-        if (lane == 0) record_walk(a, p, bits, L);
-        return;
-    }
-    RunWriter rw;
-    uint32_t* runs = ws_alloc<32>(a, grp, (unsigned long long)qe + te + 1, bh > 0);
-    const bool runs_ok = bh == 0 || runs != nullptr;
-    if (!runs_ok && lane == 0) atomicOr(a.err, (int)GMF_SWF_WORKSPACE);
-    rw.init(runs);
-    Layout16<L> lay{bits, P, W, qlen};
-    int qs = 0, ts = 0;
-    walk<L>(grp, lay, G, a, qe, te, bh, runs_ok && bh > 0, rw, qs, ts);
-    finish_cigar<L>(a, grp, p, true, rw, runs_ok, qs, ts);
 }
 
 template <int NW, bool TB, bool XD, int EM>
-__global__ void __launch_bounds__(32 * NW) sw16_coop_kernel(SwArgs a) {
-    extern __shared__ uint4 coop_ring4[];
-    uint32_t* rings = reinterpret_cast<uint32_t*>(coop_ring4);
+__global__ void __launch_bounds__(32 * NW, 16 / NW) sw16_coop_kernel(SwArgs a) {
+    extern __shared__ uint4 coop_smem[];
     __shared__ int prog[NW];
     __shared__ int cons[NW];
     __shared__ int sbest[NW][3];
@@ -867,12 +873,13 @@ __global__ void __launch_bounds__(32 * NW) sw16_coop_kernel(SwArgs a) {
     constexpr int CLS = NW == 2 ? CLS_I16_C2 : (NW == 4 ? CLS_I16_C4 : CLS_I16_C8);
     const int count = a.queue[N_CLASSES + CLS];
     const int32_t* list = a.lists + (size_t)CLS * a.n_pairs;
-    for (;;) {
-        if (threadIdx.x == 0) spair = atomicAdd(&a.queue[CLS], 1);
+    int idx = blockIdx.x;  // the first pairs go to different SMs
+    while (idx < count) {
+        sw16_coop_pair<NW, TB, XD, EM>(a, list[idx], reinterpret_cast<unsigned char*>(coop_smem), prog, cons, sbest,
+                                       &sws);
+        if (threadIdx.x == 0) spair = atomicAdd(&a.queue[CLS], 1) + (int)gridDim.x;
         __syncthreads();
-        const int idx = spair;
-        if (idx >= count) break;
-        sw16_coop_pair<NW, TB, XD, EM>(a, list[idx], rings, prog, cons, sbest, &sws);
+        idx = spair;
         __syncthreads();
     }
 }
@@ -881,7 +888,7 @@ int sw16_coop_warps(int cls) { return cls == CLS_I16_C2 ? 2 : (cls == CLS_I16_C4
 
 template <int NW, bool TB, bool XD, int EM>
 static int launch_coop(const SwArgs& a, cudaStream_t stream) {
-    const size_t smem = (size_t)NW * a.ring * sizeof(uint32_t);
+    const size_t smem = NW * group_smem_bytes(a.ring, a.tring, a.tabn);
     void (*k)(SwArgs) = sw16_coop_kernel<NW, TB, XD, EM>;
     if (smem > 48 * 1024)
         GMF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -966,15 +973,15 @@ int launch_sw_walk(const SwArgs& a, cudaStream_t stream) {
     return cuda_status(cudaGetLastError());
 }
 
-int sw16_smem_per_warp(int cls, int ring) {
+int sw16_smem_per_warp(int cls, int ring, int tring, int tabn) {
     const int L = cls == CLS_I16_L8 ? 8 : (cls == CLS_I16_L16 ? 16 : 32);
-    return (32 / L) * ring * (int)sizeof(uint32_t);
+    return (32 / L) * (int)group_smem_bytes(ring, tring, tabn);
 }
 
 template <int L, bool TB, bool XD, int EM>
 static int launch_l(const SwArgs& a, int grid, int wpb, cudaStream_t stream) {
     const int cls = L == 8 ? CLS_I16_L8 : (L == 16 ? CLS_I16_L16 : CLS_I16_L32);
-    const size_t smem = (size_t)sw16_smem_per_warp(cls, a.ring) * wpb;
+    const size_t smem = (size_t)sw16_smem_per_warp(cls, a.ring, a.tring, a.tabn) * wpb;
     void (*k)(SwArgs) = sw16_kernel<L, TB, XD, EM>;
     if (smem > 48 * 1024)
         GMF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -462,11 +462,12 @@ extern "C" int gmf_banded_sw(const gmf_pairs* pairs, const gmf_sw_params* params
     const bool xd = params->x_drop > 0;
     const int em = e_mode_of(params);
     a.defer_walk = tb ? 1 : 0;
+    a.sms = di.sms;
     std::lock_guard<std::mutex> lock(g_side_mu);
     gmf_sw_tuning tun;
     GMF_TRY(current_tuning(&tun));
-    a.l8w = tun.l8_max_w;
-    a.l16w = tun.l16_max_w;
+    a.l8w = std::min(tun.l8_max_w, L8_WMAX);
+    a.l16w = std::min(tun.l16_max_w, L16_WMAX);
     for (int i = 0; i < 3; ++i) a.cmin[i] = tun.coop_min_strips[i];
 
     const int cls_blocks = std::min((pairs->n_pairs + 255) / 256, di.sms * 4);
@@ -506,20 +507,27 @@ extern "C" int gmf_banded_sw(const gmf_pairs* pairs, const gmf_sw_params* params
         // the 8-warp class bounds each warp's lead over its reader (1024 entries
         // cover periods up to COOP_PMAX); the others hold a whole period
         ac.ring = coop_cls[c] == CLS_I16_C8 ? 1024 : ring_entries(std::min(Pmax, coop_pcap[c]) + 7);
-        if ((size_t)sw16_coop_warps(coop_cls[c]) * ac.ring * 4 > (size_t)di.smem_optin) return GMF_ERR_LIMIT;
+        ac.tring = ring_entries(std::min(Pmax, coop_pcap[c]) + 7);
+        ac.tabn = MASK_ROWS;
+        if ((size_t)sw16_coop_warps(coop_cls[c]) * sw16_smem_per_warp(CLS_I16_L32, ac.ring, ac.tring, ac.tabn) + 1024 >
+            (size_t)di.smem_optin)
+            return GMF_ERR_LIMIT;
         cudaStream_t s;
         GMF_TRY(next_stream(&s));
         GMF_TRY(launch_sw16_coop(ac, coop_cls[c], tb, xd, em, s));
     }
     // one-warp and shared-warp classes (a class only ever holds pairs up to
     // its own band limit), widest first
-    const int cls_wmax[3] = {std::min(Wmax, tun.l8_max_w), std::min(Wmax, tun.l16_max_w), Wmax};
+    const int cls_wmax[3] = {std::min(Wmax, a.l8w), std::min(Wmax, a.l16w), Wmax};
     const int lanes[3] = {8, 16, 32};
     for (int c = 2; c >= 0; --c) {
         const int L = lanes[c];
         SwArgs ac = a;
         ac.ring = ring_entries(std::max(3, sw16_period(cls_wmax[c], L) - 4 * L - 1));
-        const int wpb = warps_per_block((size_t)sw16_smem_per_warp(c, ac.ring), di, tun.warps_per_block);
+        ac.tring = ring_entries(sw16_period(cls_wmax[c], L) + 7);
+        ac.tabn = L == 32 ? MASK_ROWS : sw16_period(cls_wmax[c], L) / 4;
+        const int wpb = warps_per_block((size_t)sw16_smem_per_warp(c, ac.ring, ac.tring, ac.tabn), di,
+                                        tun.warps_per_block);
         if (wpb == 0) return GMF_ERR_LIMIT;
         const int grid = di.sms * std::max(1, 16 / wpb);
         cudaStream_t s;

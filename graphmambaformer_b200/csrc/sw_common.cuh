@@ -59,6 +59,9 @@ struct SwArgs {
     int32_t g16, m16, x16, o16, e16;  // g, and match / mismatch / open / extend divided by g
     K16 k16;                          // the 16x2 form's packed constants
     int32_t ring;                  // delay-line entries per lane group (power of two)
+    int32_t tring;                 // 16x2 form: bytes of a ring of target codes (power of two >= period + 8)
+    int32_t tabn;                  // 16x2 form: entries of a group's band mask table
+    int32_t sms;                   // SMs of the device
     unsigned long long* counters;  // [0] workspace words handed out (bump allocator)
     int32_t* queue;                // [N_CLASSES] heads, [N_CLASSES] counts
     int32_t* lists;                // N_CLASSES lists of n_pairs pair ids
@@ -474,13 +477,20 @@ __device__ void finish_cigar(const SwArgs& a, const Grp<G>& grp, int p, bool act
 // entries per warp in shared memory).
 constexpr int COOP_PMAX = 4088;
 
+// 16x2 form: most band mask table entries of a 32-lane group (the first 33
+// and last 33 chunks of a row), and the widest bands of the 8- and 16-lane
+// classes (their groups keep a table entry per chunk of a row and 4 or 2
+// groups share a warp's shared memory; wider pairs take the next class).
+constexpr int MASK_ROWS = 66;
+constexpr int L8_WMAX = 1021, L16_WMAX = 2045;
+
 // Launch helpers implemented by the kernel translation units.
 int launch_sw32(const SwArgs& a, bool tb, bool xd, int e_mode, bool queued, int grid, int wpb,
                 cudaStream_t stream);
 int launch_sw16(const SwArgs& a, int cls, bool tb, bool xd, int e_mode, int grid, int wpb,
                 cudaStream_t stream);
 int sw32_smem_per_warp(int ring);
-int sw16_smem_per_warp(int cls, int ring);
+int sw16_smem_per_warp(int cls, int ring, int tring, int tabn);
 int launch_sw16_coop(const SwArgs& a, int cls, bool tb, bool xd, int e_mode, cudaStream_t stream);
 int launch_sw_walk(const SwArgs& a, cudaStream_t stream);
 int sw16_coop_warps(int cls);
