@@ -64,3 +64,34 @@ def test_band_and_target_edges_in_every_class(params):
             assert np.array_equal(score.target_end, want.target_end), (params, l8, l16)
     finally:
         assert lib.gmf_sw_set_tuning(ctypes.byref(before)) == _native.GMF_OK
+
+
+@pytest.mark.parametrize("form", ["batched", "plain"])
+def test_walk_through_gaps_of_every_size(form):
+    """The walk copies the traceback words around its path in blocks of 32
+    rows and 32 slots and looks at 8 cells of a gap at a time: gaps around
+    those sizes, two gaps within one block, alignments that start and end at
+    block boundaries, and a score that falls near 0 on the way."""
+    from graphmambaformer_b200 import extension as ext, synth
+    from oracle import oracle
+
+    rng = np.random.default_rng(78)
+    ref = synth.random_reference(20_000, rng).astype(np.int8)
+    qs, ts, hbs = [], [], []
+    for gap in (1, 2, 7, 8, 9, 15, 16, 17, 18, 31, 32, 33, 40, 63, 64, 120):
+        for left in (30, 32, 33, 64, 95, 200):
+            for kind in range(3):
+                s = int(rng.integers(500, 15_000))
+                a, b, c = ref[s: s + left + 60], ref[s + left + 60: s + left + 60 + gap], ref[s + left + 60 + gap:
+                                                                                         s + 2 * left + 150 + gap]
+                whole, cut = np.concatenate([a, b, c]), np.concatenate([a, c])
+                if kind == 2:  # the gap back again some bases later
+                    m = len(a) + 20
+                    cut = np.concatenate([cut[:m], ref[:gap], cut[m:]])
+                qs.append(cut if kind else whole)
+                ts.append(whole if kind else cut)
+                hbs.append(150 if left % 2 else 40)
+    ps = synth.PairSet.from_lists(qs, ts, np.array(hbs, np.int32), np.zeros(len(qs), np.int32))
+    for params in ((2, 4, 4, 1, 0), (5, 4, 3, 1, 200)):
+        want = oracle.sw_batch(qs, ts, ps.half_band, ps.band_offset, *params, threads=8)
+        assert_sw_equal(ext.align_pairs(ps, ext.sw_params(*params), form=form), want, label=str(params))
