@@ -98,6 +98,13 @@ class GmfMinimizerIndex(Structure):
     ]
 
 
+class GmfSeedPrefix(Structure):
+    _fields_ = [
+        ("bits", c_int32),
+        ("first", c_void_p),
+    ]
+
+
 class GmfChainParams(Structure):
     _fields_ = [
         ("max_lookback", c_int32),
@@ -246,6 +253,12 @@ _SIGNATURES = {
                                c_void_p]),
     "gmf_seed_fill": (c_int, [POINTER(GmfMinimizerIndex), c_int32, c_void_p, c_void_p, c_int32, c_void_p,
                               c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "gmf_seed_prefix_fill": (c_int, [POINTER(GmfMinimizerIndex), c_int32, c_void_p, c_void_p]),
+    "gmf_seed_workspace_bytes": (c_size_t, [c_int32, c_int64]),
+    "gmf_seed_scan": (c_int, [POINTER(GmfMinimizerIndex), POINTER(GmfSeedPrefix), c_int32, c_void_p, c_void_p,
+                              c_int64, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
+    "gmf_seed_emit": (c_int, [POINTER(GmfMinimizerIndex), c_int32, c_void_p, c_int64, c_int32, c_void_p, c_void_p,
+                              c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "gmf_sw_get_tuning": (c_int, [POINTER(GmfSwTuning)]),
     "gmf_sw_set_tuning": (c_int, [POINTER(GmfSwTuning)]),
     "gmf_sw_test_coop_wait": (c_int, [c_int32, c_int32]),

@@ -3,8 +3,9 @@
 The index is the reference's (w, k) minimizer table (alignment/seeding.py
 L524-538: pack_kmers, hash64, minimizer_mask, KmerTable.build with
 max_occ), built once on the host by the same functions
-(``synth.MinimizerSketch`` restates them) and kept on the device.  Reads are
-seeded by ``gmf_seed_count`` / ``gmf_seed_fill``: both orientations, forward
+(``synth.MinimizerSketch`` restates them) and kept on the device with a
+prefix table over its keys.  Reads are seeded by ``gmf_seed_scan`` /
+``gmf_seed_emit``: both orientations, forward
 anchors first, reverse-complement anchors in the reverse-complemented read's
 coordinates -- what SeedingEngine.seed_read (L1056-1101) collects from
 MinimizerIndex.query before merging diagonals.
@@ -38,6 +39,19 @@ class DeviceMinimizerIndex:
         self.offsets = to_device(sk.offsets.astype(np.int64), self.device)
         self.positions = to_device(pad(sk.positions, np.int32), self.device)
         self.bytes = int(self.keys.numel() * 8 + self.offsets.numel() * 8 + self.positions.numel() * 4)
+        # about one key per bucket, so a lookup is one load of the table and one or two of keys
+        self.prefix = None
+        if 0 < self.n_keys < 2 ** 31:
+            self.prefix_bits = min(2 * self.k, 24, max(1, self.n_keys.bit_length()))
+            self.prefix = torch.empty((1 << self.prefix_bits) + 1, dtype=torch.int32, device=self.device)
+            s = torch.cuda.current_stream(self.device)
+            bind(self.device, int(s.cuda_stream))
+            idx = self.c()
+            _native.check("gmf_seed_prefix_fill", _native.lib().gmf_seed_prefix_fill(
+                ctypes.byref(idx), self.prefix_bits, ctypes.c_void_p(self.prefix.data_ptr()),
+                ctypes.c_void_p(int(s.cuda_stream))))
+            s.synchronize()  # other streams read it
+            self.bytes += int(self.prefix.numel() * 4)
 
     def c(self) -> _native.GmfMinimizerIndex:
         return _native.GmfMinimizerIndex(self.k, self.w, self.n_keys, self.keys.data_ptr(), self.offsets.data_ptr(),
@@ -57,27 +71,31 @@ class DeviceMinimizerIndex:
         # every allocation and torch op on the caller's stream: the library's
         # kernels run there, and a worker's stream is not ordered with the
         # thread's default stream
+        total_codes = int(codes_d.numel())
+        pre = _native.GmfSeedPrefix(self.prefix_bits, self.prefix.data_ptr()) if self.prefix is not None else None
+        both = 1 if both_strands else 0
+        lib = _native.lib()
         with torch.cuda.stream(s):
-            counts = torch.empty(max(2 * n_reads, 1), dtype=torch.int64, device=self.device)
-            _native.check("gmf_seed_count", _native.lib().gmf_seed_count(
-                ctypes.byref(idx), n_reads, vp(codes_d.data_ptr()), vp(read_off_d.data_ptr()),
-                1 if both_strands else 0, vp(counts.data_ptr()), vp(sp)))
-            aoff = torch.zeros(2 * n_reads + 1, dtype=torch.int64, device=self.device)
-            if n_reads:
-                torch.cumsum(counts[: 2 * n_reads], 0, out=aoff[1:])
+            need = int(lib.gmf_seed_workspace_bytes(n_reads, total_codes))
+            ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
+            off = torch.empty(3 * n_reads + 4, dtype=torch.int64, device=self.device)
+            aoff, roff, totals = off[: 2 * n_reads + 1], off[2 * n_reads + 1: 3 * n_reads + 2], off[3 * n_reads + 2:]
+            _native.check("gmf_seed_scan", lib.gmf_seed_scan(
+                ctypes.byref(idx), ctypes.byref(pre) if pre is not None else None, n_reads, vp(codes_d.data_ptr()),
+                vp(read_off_d.data_ptr()), total_codes, both, vp(aoff.data_ptr()), vp(roff.data_ptr()),
+                vp(totals.data_ptr()), vp(ws.data_ptr()), ws.numel(), vp(sp)))
             # the total sizes the outputs; the largest read is checked against the chaining limit (one
             # host round trip for both)
-            per_read = (counts[0: 2 * n_reads: 2] + counts[1: 2 * n_reads: 2]).max() if n_reads else counts[0] * 0
-            total, most = (int(x) for x in torch.stack([aoff[-1], per_read]).cpu().tolist())
+            total, most = (int(x) for x in totals.cpu().tolist())
             i32 = dict(dtype=torch.int32, device=self.device)
             out = dict(read_pos=torch.empty(max(total, 1), **i32), ref_pos=torch.empty(max(total, 1), **i32),
                        length=torch.empty(max(total, 1), **i32),
                        strand=torch.empty(max(total, 1), dtype=torch.int8, device=self.device))
-            _native.check("gmf_seed_fill", _native.lib().gmf_seed_fill(
-                ctypes.byref(idx), n_reads, vp(codes_d.data_ptr()), vp(read_off_d.data_ptr()),
-                1 if both_strands else 0, vp(aoff.data_ptr()), vp(out["read_pos"].data_ptr()),
-                vp(out["ref_pos"].data_ptr()), vp(out["length"].data_ptr()), vp(out["strand"].data_ptr()), vp(sp)))
-            out["read_off"] = aoff[::2].contiguous()
+            _native.check("gmf_seed_emit", lib.gmf_seed_emit(
+                ctypes.byref(idx), n_reads, vp(read_off_d.data_ptr()), total_codes, both, vp(aoff.data_ptr()),
+                vp(out["read_pos"].data_ptr()), vp(out["ref_pos"].data_ptr()), vp(out["length"].data_ptr()),
+                vp(out["strand"].data_ptr()), vp(ws.data_ptr()), ws.numel(), vp(sp)))
+            out["read_off"] = roff
         out["n_anchors"] = total
         out["max_read_anchors"] = most
         return out

@@ -159,7 +159,7 @@ class BatchAligner:
         reads_d = up("reads", codes, s)
         pad = lambda x, dt: x if len(x) else np.zeros(1, dt)  # noqa: E731
         if anchors is None:  # device seeding: both orientations, forward anchors first
-            sd = self.index.seed_device(reads_d, up("roff", roff, s), R, True, stream=s)
+            sd = self.index.seed_device(reads_d[: len(codes)], up("roff", roff, s), R, True, stream=s)
             ro, rp, fp, ln, st = sd["read_off"], sd["read_pos"], sd["ref_pos"], sd["length"], sd["strand"]
             A = int(sd["n_anchors"])
             per_read = int(sd["max_read_anchors"])

@@ -216,6 +216,40 @@ int gmf_seed_fill(const gmf_minimizer_index* index, int32_t n_reads, const int8_
                   int32_t* read_pos, int32_t* ref_pos, int32_t* length, int8_t* strand,
                   gmf_stream_t stream);
 
+/* The same two passes with a workspace, for batches of reads of any length:
+ * every 512-base tile of a read is scanned by a block of its own, both
+ * orientations at once, and the lookups are done once.
+ *
+ * Optional lookup table over the index keys: first[b] is the first key of
+ * bucket b = key >> (2 * k - bits), first[2^bits] = n_keys (device, int32;
+ * n_keys < 2^31, bits <= 2 * k).  gmf_seed_prefix_fill writes it. */
+typedef struct {
+    int32_t bits;
+    const int32_t* first; /* 2^bits + 1 entries */
+} gmf_seed_prefix;
+
+int gmf_seed_prefix_fill(const gmf_minimizer_index* index, int32_t bits, int32_t* first, gmf_stream_t stream);
+
+/* total_codes: host value >= read_off[n_reads] (codes beyond it are not read
+ * and find no anchors). */
+size_t gmf_seed_workspace_bytes(int32_t n_reads, int64_t total_codes);
+
+/* Scan: anchor_off[2 * n_reads + 1] receives the anchor offsets (per read
+ * forward, then reverse complement; the reverse ones empty when both_strands
+ * is 0), read_anchor_off[n_reads + 1] (may be NULL) those of the reads,
+ * totals[0] their number and totals[1] the largest read's.  prefix may be
+ * NULL. */
+int gmf_seed_scan(const gmf_minimizer_index* index, const gmf_seed_prefix* prefix, int32_t n_reads,
+                  const int8_t* codes, const int64_t* read_off, int64_t total_codes, int32_t both_strands,
+                  int64_t* anchor_off, int64_t* read_anchor_off, int64_t* totals, void* workspace,
+                  size_t workspace_bytes, gmf_stream_t stream);
+
+/* Emit: the anchors of a scan with the same arguments and workspace, as
+ * gmf_seed_fill writes them. */
+int gmf_seed_emit(const gmf_minimizer_index* index, int32_t n_reads, const int64_t* read_off, int64_t total_codes,
+                  int32_t both_strands, const int64_t* anchor_off, int32_t* read_pos, int32_t* ref_pos,
+                  int32_t* length, int8_t* strand, void* workspace, size_t workspace_bytes, gmf_stream_t stream);
+
 /* Scheduling knobs of the batched form (per device, process-wide).  They
  * decide which kernel shape aligns which pair and how the kernels overlap;
  * results never depend on them.  graphmambaformer_b200.autotune times
