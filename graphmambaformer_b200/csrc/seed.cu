@@ -215,10 +215,11 @@ __global__ void __launch_bounds__(SEED_THREADS) seed_kernel(SeedArgs a) {
 // looks the selected k-mers up in the index once, through a prefix table (one
 // load instead of ~20 dependent ones).  The selected positions and their keys
 // stay in the workspace; the emit pass only expands them.
-// What bounds it now is the hash and minimum arithmetic (about 250
-// instructions a position) and, for small batches, the four launches.
-// Measured on one B200, 1,024 reads of 150-20,000 bases on a 1.2 Mb
-// reference: SEED_SCAN us + SEED_EMIT us against 541 + 543 us.
+// What bounds it now is the hash and minimum arithmetic (about 280
+// instructions a position, 600 with the k-mers packed base by base) and, for
+// small batches, the four launches.  Measured on one B200, 1,024 reads of
+// 150-20,000 bases on a 1.2 Mb reference: SEED_SCAN us + 23 us (emit) against
+// 541 + 543 us.
 // ---------------------------------------------------------------------------
 constexpr int TILE = 512;
 constexpr int TILE_THREADS = 256;
@@ -284,9 +285,39 @@ __device__ __forceinline__ long long find_key(const TileArgs& a, long long key) 
     return -1;
 }
 
+// The packed k-mers at base x of a tile whose codes are all A, C, G or T:
+// forward from words that hold the first base in their top bits, reverse
+// complement from words of complemented digits with the first base in their
+// low bits.
+constexpr int TILE_WORDS = (TILE_HASHES + SEED_MAX_K) / 16 + 4;
+__device__ __forceinline__ ulonglong2 kmer_pair(const uint32_t* fw, const uint32_t* rc, int x, int k) {
+    const int w = x >> 4, sh = 2 * (x & 15);
+    const uint32_t a0 = __funnelshift_l(fw[w + 1], fw[w], sh), a1 = __funnelshift_l(fw[w + 2], fw[w + 1], sh);
+    const uint32_t b0 = __funnelshift_r(rc[w], rc[w + 1], sh), b1 = __funnelshift_r(rc[w + 1], rc[w + 2], sh);
+    return make_ulonglong2(((unsigned long long)a0 << 32 | a1) >> (64 - 2 * k),
+                           ((unsigned long long)b1 << 32 | b0) & ((1ull << (2 * k)) - 1ull));
+}
+
+// The same for any codes (1..4 are A, C, G, T; a digit above 3 makes the k-mer
+// invalid, packed to 0).
+__device__ __forceinline__ ulonglong2 kmer_pair_any(const int8_t* code, int k, bool& bad) {
+    unsigned long long f = 0, c = 0;
+    bad = false;
+    for (int o = 0; o < k; ++o) {
+        const int dg = (int)code[o] - 1;
+        bad |= dg > 3;
+        f = f * 4 + (unsigned long long)(long long)dg;
+        // reverse_complement_codes: 1..4 -> 4..1, others kept
+        const int dc = (unsigned)dg < 4u ? 3 - dg : dg;
+        c += (unsigned long long)(long long)dc << (2 * o);
+    }
+    return bad ? make_ulonglong2(0ull, 0ull) : make_ulonglong2(f, c);
+}
+
 __global__ void __launch_bounds__(TILE_THREADS) seed_tile_kernel(TileArgs a) {
     __shared__ ulonglong2 s_a[TILE_HASHES], s_b[TILE_HASHES];  // (forward, reverse) hashes, minima, maxima
-    __shared__ longlong2 s_key[TILE];                          // packed k-mers of the tile
+    __shared__ ulonglong2 s_hash[TILE];                        // the tile's own hashes
+    __shared__ uint32_t s_fw[TILE_WORDS], s_rc[TILE_WORDS];    // digits, 16 to a word (see kmer_pair)
     __shared__ int8_t s_code[TILE_HASHES + SEED_MAX_K];
     __shared__ bool s_valid[TILE];
     __shared__ unsigned short s_pos[2 * TILE];
@@ -318,24 +349,34 @@ __global__ void __launch_bounds__(TILE_THREADS) seed_tile_kernel(TileArgs a) {
         const int n_win = m - ww + 1;
         // hashed positions [h0, h1): the windows that cover the tile
         const int h0 = max(t0 - ww + 1, 0), h1 = min(t1 + ww - 1, m), H = h1 - h0;
-        for (int x = tid; x < H + k - 1; x += TILE_THREADS) s_code[x] = a.s.codes[r0 + h0 + x];
-        __syncthreads();
-        for (int x = tid; x < H; x += TILE_THREADS) {
-            unsigned long long f = 0, c = 0;
-            bool bad = false;
-            for (int o = 0; o < k; ++o) {
-                const int dg = (int)s_code[x + o] - 1;
-                bad |= dg > 3;
-                f = f * 4 + (unsigned long long)(long long)dg;
-                // reverse_complement_codes: 1..4 -> 4..1, others kept
-                const int dc = (unsigned)dg < 4u ? 3 - dg : dg;
-                c += (unsigned long long)(long long)dc << (2 * o);
+        bool other = false;
+        for (int x = tid; x < H + k - 1; x += TILE_THREADS) {
+            const int8_t c = a.s.codes[r0 + h0 + x];
+            s_code[x] = c;
+            other |= c < 1 || c > 4;
+        }
+        const bool plain = !__syncthreads_or(other);
+        if (plain) {
+            for (int x = tid; x < (H + k - 1 + 15) / 16 + 2; x += TILE_THREADS) {
+                uint32_t f = 0, c = 0;
+                for (int o = 0; o < 16; ++o) {
+                    const uint32_t dg = 16 * x + o < H + k - 1 ? (uint32_t)(s_code[16 * x + o] - 1) : 0u;
+                    f |= dg << (30 - 2 * o);
+                    c |= (3u - dg) << (2 * o);
+                }
+                s_fw[x] = f;
+                s_rc[x] = c;
             }
-            if (bad) f = c = 0;
-            s_a[x] = make_ulonglong2(mm_hash64(f), mm_hash64(c));
+            __syncthreads();
+        }
+        for (int x = tid; x < H; x += TILE_THREADS) {
+            bool bad = false;
+            const ulonglong2 key = plain ? kmer_pair(s_fw, s_rc, x, k) : kmer_pair_any(s_code + x, k, bad);
+            const ulonglong2 h = make_ulonglong2(mm_hash64(key.x), mm_hash64(key.y));
+            s_a[x] = h;
             const int p = h0 + x;
             if (p >= t0 && p < t1) {
-                s_key[p - t0] = make_longlong2((long long)f, (long long)c);
+                s_hash[p - t0] = h;
                 s_valid[p - t0] = !bad;
             }
         }
@@ -392,10 +433,9 @@ __global__ void __launch_bounds__(TILE_THREADS) seed_tile_kernel(TileArgs a) {
             bool sf = false, sr = false;
             if (t0 + x < t1) {
                 if (s_valid[x]) {
-                    const longlong2 key = s_key[x];
-                    const ulonglong2 mx = src[t0 + x - h0];
-                    sf = mx.x == mm_hash64((unsigned long long)key.x);
-                    sr = both && mx.y == mm_hash64((unsigned long long)key.y);
+                    const ulonglong2 mx = src[t0 + x - h0], h = s_hash[x];
+                    sf = mx.x == h.x;
+                    sr = both && mx.y == h.y;
                 }
             }
             bal[0][e] = __ballot_sync(gmf::FULL_MASK, sf);
@@ -436,8 +476,10 @@ __global__ void __launch_bounds__(TILE_THREADS) seed_tile_kernel(TileArgs a) {
             const int o = x < n_all[0] ? 0 : 1;
             const int n = o ? x - n_all[0] : x;
             const int p = s_pos[o * TILE + n];
-            const longlong2 key = s_key[p];
-            const long long at = find_key(a, o ? key.y : key.x);
+            bool bad;
+            const ulonglong2 key =
+                plain ? kmer_pair(s_fw, s_rc, t0 + p - h0, k) : kmer_pair_any(s_code + (t0 + p - h0), k, bad);
+            const long long at = find_key(a, (long long)(o ? key.y : key.x));
             const long long slot_o = (2 * slot + o) * TILE + n;
             a.pos[slot_o] = (unsigned short)p;
             a.at[slot_o] = (int32_t)at;
