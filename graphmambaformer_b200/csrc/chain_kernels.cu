@@ -114,6 +114,7 @@ struct SortArgs {
     int32_t* n_minus;
     int32_t* read_end_s;
     int32_t* ref_end_s;
+    int32_t* len_s;            // sorted lengths (workspace), or null
     unsigned long long* gkey;  // workspace: 2 * n_anchors keys (large reads)
     int* gidx;                 // workspace: 2 * n_anchors indices
     int smem_elems;
@@ -184,6 +185,7 @@ __global__ void __launch_bounds__(256) chain_sort_kernel(SortArgs a) {
     for (int x = threadIdx.x; x < m; x += blockDim.x) {
         const unsigned long long k = key[x];
         a.perm[a0 + x] = idx[x];
+        if (a.len_s) a.len_s[a0 + x] = a.length[a0 + idx[x]];
         a.ref_end_s[a0 + x] = (int32_t)((k >> 31) & 0x7fffffffu);
         a.read_end_s[a0 + x] = (int32_t)(k & 0x7fffffffu);
     }
@@ -207,6 +209,7 @@ struct DpArgs {
     const int32_t* ref_end;
     const double* weight;    // NULL: anchor length (reads mode), via length_s
     const int32_t* length;   // original lengths (reads mode, weight == NULL)
+    const int32_t* len_s;    // sorted lengths, or null: length[perm[]]
     const int32_t* perm;     // reads mode
     const double* bonus;
     int32_t lookback;
@@ -216,6 +219,7 @@ struct DpArgs {
     double* f;
     int32_t* parent;
     int32_t ring;            // ring entries per warp (power of two > lookback)
+    bool near;               // sorted by this call with lengths as weights: at most GMF_MAX_READ_ANCHORS a segment
     int64_t cap;             // reads mode: anchors f / parent hold (-1: caller-sized)
 };
 
@@ -335,7 +339,7 @@ __device__ __forceinline__ void dp_load_slot(const DpArgs& a, int64_t st, int64_
         if (WEIGHT) {
             w = a.weight[gi];
         } else {
-            wl = a.length[r0 + a.perm[gi]];
+            wl = a.len_s ? a.len_s[gi] : a.length[r0 + a.perm[gi]];
             w = (double)wl;
         }
     } else {
@@ -441,6 +445,202 @@ __global__ void __launch_bounds__(128) chain_dp_bcast_kernel(DpArgs a) {
             dp_load_slot<WEIGHT>(a, st, r0, base + 32 * K + lane, n, q[K - 1], rr[K - 1], w[K - 1], wl[K - 1]);
             best[K - 1] = -INFINITY;
             bj[K - 1] = -1;
+        }
+    }
+}
+
+// The same recurrence with the nearest predecessors first, for sorted reads
+// whose weights are their lengths (no bonus).  A group of G lanes runs one
+// segment, G anchors (a block) at a time: every lane first computes, for its
+// own anchor, advance and penalty against the NEAR nearest predecessors --
+// nothing of that depends on f -- and then all lanes of the group step
+// through the block's anchors together, each anchor scoring its NEAR nearest
+// predecessors from shared memory, oldest first, so that the first maximum
+// wins and only two additions and a compare lie between f[i-1] and f[i].
+//
+// Predecessors beyond the nearest are scored only when they could matter:
+// none of them scores more than (the largest f among them) + w_i - (the
+// smallest penalty), float64 rounding being monotone, and on a chain f grows
+// by several units per anchor, so that bound (with the largest f of all older
+// anchors) nearly always lies below the best near candidate.  Otherwise the
+// group's lanes score the rest of the window, oldest first; an older
+// candidate wins a tie.
+//
+// What bounds it is that chain, one segment being one serial scan: the
+// broadcast form above scores the whole window (98 instructions and ~480
+// cycles an anchor for a window of 50, 8 blocks of 32 for 200).  A pull form
+// with one candidate per lane and two warp reductions per anchor took 100
+// instructions and 380 cycles.  Measured on one B200, DP kernel alone: one
+// 15 kb HiFi read 675 -> 268 us, 5,000 of them 1,874 -> 925 us (window 50),
+// 1,000 reads of 50-100 kb 5,011 -> 1,048 us (window 200).
+//
+__device__ __forceinline__ double int_to_double(int x) {  // exact: one add instead of a conversion
+    return __hiloint2double(0x43300000, x ^ (int)0x80000000) - 4503601774854144.0;  // 2^52 + 2^31
+}
+
+// Advance and penalty of a predecessor (dq, dr behind the anchor), infinite
+// penalty when the pair is out of range.
+__device__ __forceinline__ double2 dp_pair(int dq, int dr, int wl, bool in, unsigned mg,
+                                           const double* __restrict__ lut) {
+    const bool ok = in && (unsigned)(dq - 1) < mg && (unsigned)(dr - 1) < mg;
+    const int mn = dq < dr ? dq : dr;
+    const unsigned gap = (unsigned)(dr > dq ? dr - dq : dq - dr);
+    const double pen = __ldg(&lut[gap < mg ? gap : mg]);
+    return make_double2(ok ? int_to_double(mn < wl ? mn : wl) : 0.0, ok ? pen : INFINITY);
+}
+
+constexpr int NEAR = 4;
+constexpr int NEAR_MAX_GAP = 16384;  // every block reads the whole penalty table once for its minimum
+constexpr int NEAR_WARPS = 2;        // per block: small blocks spread the long segments over the SMs
+
+__host__ __device__ inline size_t near_smem_bytes(int G, int ring) {  // per group
+    return (size_t)G * (NEAR * 16 + 16 + 8) + (size_t)ring * 16;
+}
+
+template <int G>
+__global__ void __launch_bounds__(32 * NEAR_WARPS) chain_dp_near_kernel(DpArgs a) {
+    extern __shared__ double2 near_smem[];
+    __shared__ double s_min[NEAR_WARPS];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, gl = lane & (G - 1);
+    constexpr int GPW = 32 / G, UNROLL = 8;
+    const int R = a.ring, rm = R - 1;  // R is a multiple of G: a block's entries never wrap
+    unsigned char* sm = reinterpret_cast<unsigned char*>(near_smem) +
+                        (size_t)(threadIdx.x / G) * near_smem_bytes(G, R);
+    double2* s_pair = reinterpret_cast<double2*>(sm);              // [G][NEAR] (advance, penalty), nearest first
+    double2* s_w = s_pair + G * NEAR;                              // [G] (weight, weight - smallest penalty + slack)
+    double* s_f = reinterpret_cast<double*>(s_w + G);              // ring of f
+    int2* s_qr = reinterpret_cast<int2*>(s_f + R);                 // ring of (read_end, ref_end)
+    int* s_p = reinterpret_cast<int*>(s_qr + R);                   // [G] age of a predecessor beyond the nearest, else 0
+    const int lb = a.lookback > 1 ? a.lookback : 1;
+    const unsigned mg = a.max_gap > 0 ? (unsigned)a.max_gap : 0u;
+    const double* __restrict__ lut = a.lut;
+    // smallest penalty a candidate can take
+    double min_pen = INFINITY;
+#pragma unroll 8
+    for (unsigned x = threadIdx.x; x <= mg; x += 32 * NEAR_WARPS) min_pen = fmin(min_pen, __ldg(&lut[x]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) min_pen = fmin(min_pen, __shfl_xor_sync(FULL_MASK, min_pen, o));
+    if (lane == 0) s_min[wib] = min_pen;
+    __syncthreads();
+    for (int x = 0; x < NEAR_WARPS; ++x) min_pen = fmin(min_pen, s_min[x]);
+
+    const int n_reads = a.n_segments >> 1;
+    const int n_groups = gridDim.x * NEAR_WARPS * GPW;
+    for (int g0 = (blockIdx.x * NEAR_WARPS + wib) * GPW; g0 < a.n_segments; g0 += n_groups) {
+        const int g = g0 + lane / G;
+        int64_t st = 0, r0 = 0;
+        int n = 0;
+        if (g < a.n_segments) {
+            // every read's longer strand first, then the shorter ones
+            const int r = g < n_reads ? g : g - n_reads;
+            const int minus_longer = a.n_minus[r] > a.n_plus[r] ? 1 : 0;
+            seg_range(a, 2 * r + (g < n_reads ? minus_longer : 1 - minus_longer), st, n);
+            r0 = a.read_off[r];
+        }
+        const int blocks = __reduce_max_sync(FULL_MASK, (n + G - 1) / G);
+        double f1 = 0.0, f2 = 0.0, f3 = 0.0, f4 = 0.0;  // f of the four anchors before
+        double older = -INFINITY;                       // largest f before those
+        int q, r, wl;
+        double unused;
+        dp_load_slot<false>(a, st, r0, gl, n, q, r, unused, wl);
+        for (int b = 0; b < blocks; ++b) {
+            const int base = b * G, mine = base + gl;
+            double* f_at = s_f + (base & rm);
+            __syncwarp();
+            s_qr[mine & rm] = make_int2(q, r);
+            s_p[gl] = 0;
+            __syncwarp();
+#pragma unroll
+            for (int d = 1; d <= NEAR; ++d) {
+                const int2 c = s_qr[(mine - d) & rm];
+                s_pair[gl * NEAR + d - 1] = dp_pair(q - c.x, r - c.y, wl, d <= mine && d <= lb && mine < n, mg, lut);
+            }
+            {
+                // the slack covers the candidates' two roundings: |f| < 2^14 anchors * 2^31
+                const double w = int_to_double(wl);
+                s_w[gl] = make_double2(w, mine < n ? w - min_pen + 0.015625 : -INFINITY);
+            }
+            dp_load_slot<false>(a, st, r0, mine + G, n, q, r, unused, wl);  // the next block
+            __syncwarp();
+            double2 p1 = s_pair[0], p2 = s_pair[1], p3 = s_pair[2], p4 = s_pair[3], w = s_w[0];
+            for (int u0 = 0; u0 < G; u0 += UNROLL) {
+                const double2* pair_at = s_pair + u0 * NEAR;
+#pragma unroll
+                for (int v = 0; v < UNROLL; ++v) {
+                    const double2 wi = w;
+                    const double c4 = __dsub_rn(__dadd_rn(f4, p4.x), p4.y), c3 = __dsub_rn(__dadd_rn(f3, p3.x), p3.y);
+                    const double c2 = __dsub_rn(__dadd_rn(f2, p2.x), p2.y), c1 = __dsub_rn(__dadd_rn(f1, p1.x), p1.y);
+                    // the next anchor's pairs, ahead of this one's result (the block's last step reads its own again)
+                    const int nv = v + 1 < UNROLL || u0 + UNROLL < G ? v + 1 : v;
+                    p1 = pair_at[nv * NEAR];
+                    p2 = pair_at[nv * NEAR + 1];
+                    p3 = pair_at[nv * NEAR + 2];
+                    p4 = pair_at[nv * NEAR + 3];
+                    w = s_w[u0 + nv];
+                    const double x = c4 > wi.x ? c4 : wi.x, y = c2 > c3 ? c2 : c3;
+                    const double z = y > x ? y : x;
+                    double best = c1 > z ? c1 : z;
+                    if (!(older + wi.y < best)) {
+                        // an older predecessor may score as much: the rest of the window, oldest first
+                        const int u = u0 + v, i = base + u;
+                        const int lim = lb < i ? lb : i;
+                        const int2 me = s_qr[i & rm];
+                        double bs = 0.0;
+                        int ba = 0;
+                        for (int t = lim > NEAR ? (lim - NEAR - 1) / G : -1; t >= 0; --t) {
+                            const int ag = NEAR + 1 + t * G + gl;
+                            if (ag <= lim) {
+                                const int2 c = s_qr[(i - ag) & rm];
+                                const int dq = me.x - c.x, dr = me.y - c.y;
+                                if ((unsigned)(dq - 1) < mg && (unsigned)(dr - 1) < mg) {
+                                    const double mn = int_to_double(dq < dr ? dq : dr);
+                                    const double sc = __dsub_rn(__dadd_rn(s_f[(i - ag) & rm], mn < wi.x ? mn : wi.x),
+                                                                __ldg(&lut[dr > dq ? dr - dq : dq - dr]));
+                                    if (sc > wi.x && (ba == 0 || sc > bs)) {
+                                        bs = sc;
+                                        ba = ag;
+                                    }
+                                }
+                            }
+                        }
+                        const unsigned gm = G == 32 ? FULL_MASK : ((1u << (G & 31)) - 1u) << (lane & ~(G - 1));
+#pragma unroll
+                        for (int o = G / 2; o > 0; o >>= 1) {
+                            const double os = __shfl_xor_sync(gm, bs, o);
+                            const int oa = __shfl_xor_sync(gm, ba, o);
+                            if (oa && (ba == 0 || os > bs || (os == bs && oa > ba))) {
+                                bs = os;
+                                ba = oa;
+                            }
+                        }
+                        if (ba && bs >= best) {
+                            best = bs;
+                            s_p[u] = ba;
+                        }
+                    }
+                    older = f4 > older && base + u0 + v >= NEAR ? f4 : older;
+                    f_at[u0 + v] = best;
+                    f4 = f3;
+                    f3 = f2;
+                    f2 = f1;
+                    f1 = best;
+                }
+            }
+            __syncwarp();
+            if (mine < n) {
+                // the predecessor: an older one, or the oldest near one that gives the score
+                const double fi = f_at[gl];
+                int age = s_p[gl];
+                if (!age && fi > s_w[gl].x) {
+#pragma unroll
+                    for (int d = 1; d <= NEAR; ++d) {
+                        const double2 p = s_pair[gl * NEAR + d - 1];
+                        if (__dsub_rn(__dadd_rn(s_f[(mine - d) & rm], p.x), p.y) == fi) age = d;
+                    }
+                }
+                a.f[st + mine] = fi;
+                a.parent[st + mine] = age ? mine - age : -1;
+            }
         }
     }
 }
@@ -909,7 +1109,7 @@ int peel_smem_elems() { return 2048; }
 
 size_t sort_smem_bytes(int elems) { return (size_t)elems * (sizeof(unsigned long long) + sizeof(int)); }
 
-int launch_sort(const gmf_anchor_batch* an, const gmf_sorted_anchors* so, unsigned long long* gkey,
+int launch_sort(const gmf_anchor_batch* an, const gmf_sorted_anchors* so, int32_t* len_s, unsigned long long* gkey,
                 int* gidx, int64_t cap, int64_t key_cap, int* err, cudaStream_t stream) {
     SortArgs s;
     s.n_reads = an->n_reads;
@@ -923,6 +1123,7 @@ int launch_sort(const gmf_anchor_batch* an, const gmf_sorted_anchors* so, unsign
     s.n_minus = so->n_minus;
     s.read_end_s = so->read_end;
     s.ref_end_s = so->ref_end;
+    s.len_s = len_s;
     s.gkey = gkey;
     s.gidx = gidx;
     s.smem_elems = sort_smem_elems();
@@ -953,9 +1154,30 @@ int launch_dp_bcast(const DpArgs& d, int n_segments, cudaStream_t stream) {
     return cuda_status(cudaGetLastError());
 }
 
+template <int G>
+int launch_dp_near(DpArgs d, int n_segments, cudaStream_t stream) {
+    const int lb = d.lookback > 1 ? d.lookback : 1;
+    constexpr int GPB = 32 * NEAR_WARPS / G;
+    d.ring = next_pow2((lb > NEAR ? lb : NEAR) + G);
+    const size_t smem = GPB * near_smem_bytes(G, d.ring);
+    GMF_CUDA_TRY(cudaFuncSetAttribute(chain_dp_near_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+    const int blocks = (n_segments + GPB - 1) / GPB;
+    if (blocks > 0) chain_dp_near_kernel<G><<<blocks, 32 * NEAR_WARPS, smem, stream>>>(d);
+    return cuda_status(cudaGetLastError());
+}
+
 int launch_dp(DpArgs d, int n_segments, cudaStream_t stream) {
     d.n_segments = n_segments;
     int lb = d.lookback > 1 ? d.lookback : 1;
+    // Sorted reads with their lengths as weights: near predecessors first.  A warp for two segments from two
+    // long segments per scheduler on (592 on the chip; half the segments are the reads' short strands), if
+    // their rings are small.  5,000 reads of 15 kb, whole chain call: 4.19 ms with 32 lanes, 3.87 with 16,
+    // 3.96 with 8; 1,000 reads of 75 kb: 5.75, 5.99, 6.80 ms.
+    if (d.near) {
+        if (n_segments > 2 * 2 * 592 && lb <= 496) return launch_dp_near<16>(d, n_segments, stream);
+        return launch_dp_near<32>(d, n_segments, stream);
+    }
     // windows up to 224 predecessors: lanes own anchors, K = ceil(lb/32) + 1
     // blocks of 32 in registers
     switch ((lb + 31) / 32 + 1) {
@@ -1032,7 +1254,7 @@ extern "C" int gmf_chain_sort(const gmf_anchor_batch* an, const gmf_sorted_ancho
         gkey = nullptr;
     }
     GMF_CUDA_TRY(cudaMemsetAsync(err, 0, 4, (cudaStream_t)stream));
-    return launch_sort(an, so, gkey, gidx, -1, (int64_t)A, err, (cudaStream_t)stream);
+    return launch_sort(an, so, nullptr, gkey, gidx, -1, (int64_t)A, err, (cudaStream_t)stream);
 }
 
 extern "C" size_t gmf_chain_workspace_bytes(int32_t n_reads, int64_t n_anchors) {
@@ -1121,7 +1343,7 @@ extern "C" int gmf_chain_batch(const gmf_anchor_batch* an, const gmf_chain_param
     GMF_CUDA_TRY(cudaMemsetAsync(err, 0, 256, stream));
     int st;
     if (!sorted_in) {
-        st = launch_sort(an, &so, gkey, gidx, (int64_t)A, (int64_t)A, err, stream);
+        st = launch_sort(an, &so, mem_tmp, gkey, gidx, (int64_t)A, (int64_t)A, err, stream);
         if (st) return st;
     }
     DpArgs d{};
@@ -1132,6 +1354,7 @@ extern "C" int gmf_chain_batch(const gmf_anchor_batch* an, const gmf_chain_param
     d.ref_end = so.ref_end;
     d.weight = sorted_weight;
     d.length = an->length;
+    d.len_s = sorted_in ? nullptr : mem_tmp;  // the sort left them where the peel will keep its members
     d.perm = so.perm;
     d.bonus = sorted_bonus;
     d.lookback = cp->max_lookback;
@@ -1141,6 +1364,7 @@ extern "C" int gmf_chain_batch(const gmf_anchor_batch* an, const gmf_chain_param
     d.f = f;
     d.parent = parent;
     d.cap = (int64_t)A;
+    d.near = !sorted_in && cp->max_gap <= NEAR_MAX_GAP;
     st = launch_dp(d, 2 * an->n_reads, stream);
     if (st) return st;
 
