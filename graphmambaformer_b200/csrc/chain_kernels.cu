@@ -14,12 +14,13 @@
 // float64 add / subtract / compare in the reference's order and the results
 // are bit-identical.
 //
-// Layout: one CTA per read for sort and peel/select (shared-memory bitonic
-// sort of 64-bit keys + 32-bit tie index; reads too large for shared memory
-// sort in their own workspace range), one warp per (read, strand) segment for
-// the DP: lanes own anchors and each finished score is broadcast to the
-// window (up to 224 predecessors), or, for wider windows, the window sits in
-// a shared-memory ring and a warp reduction picks each anchor's predecessor.
+// Layout: one CTA per read for sort (a radix sort in shared memory) and
+// peel/select, half a warp or a warp per (read, strand) segment for the DP of
+// sorted reads: the nearest predecessors first, the rest of the window when
+// it could matter.  Segments with weights or bonuses of their own take a warp
+// whose lanes own anchors, each finished score broadcast to the window (up to
+// 224 predecessors), or, for wider windows, the window sits in a shared-memory
+// ring and a warp reduction picks each anchor's predecessor.
 
 #include <float.h>
 
@@ -115,83 +116,256 @@ struct SortArgs {
     int32_t* read_end_s;
     int32_t* ref_end_s;
     int32_t* len_s;            // sorted lengths (workspace), or null
-    unsigned long long* gkey;  // workspace: 2 * n_anchors keys (large reads)
-    int* gidx;                 // workspace: 2 * n_anchors indices
-    int smem_elems;
     int64_t cap;               // anchors the sorted outputs can hold (-1: caller-sized)
-    int64_t key_cap;           // anchors gkey / gidx cover (2 entries each)
+    int64_t key_cap;           // anchors the caller's workspace covers (reads beyond SORT_CAP need it)
     int* err;
 };
 
-__global__ void __launch_bounds__(256) chain_sort_kernel(SortArgs a) {
-    extern __shared__ unsigned long long sm_keys[];
-    const int r = blockIdx.x;
-    if (r >= a.n_reads) return;
+// Radix sort of a read's anchors in shared memory: 16-bit indices by 8-bit
+// digits of a 32-bit key, least significant first.  Every pass is stable, so
+// equal keys keep the input order, which is the reference's last tie-breaker.
+// The key is the strand and ref_end (less the read's smallest); read_end needs
+// passes of its own only when the anchors do not come in (strand, read_end)
+// order, which is how seeding writes them.  A pass ranks each warp's run of
+// anchors row by row of 32 (lanes of equal digit found by a match), turns the
+// warps' digit counts into offsets, and scatters the indices.
+//
+// What bounds it is the latency of a pass's rows; a bitonic sort of (key,
+// index) pairs took 78 stages for 4,096 keys (199,000 warp instructions for a
+// 15 kb read's 2,700 anchors) and went through global memory beyond that.
+// Measured on one B200: one 15 kb read 89 -> 28 us, 5,000 of them 1,275
+// -> 338 us, 1,000 reads of 10,000 anchors 2,172 -> 296 us.
+constexpr int SORT_CAP = 4096;      // anchors a 256-thread block sorts; larger reads take 1,024 threads
+constexpr int SORT_CAP_BIG = 16384;
+constexpr int SORT_ROWS = 16;       // rows of 32 a warp takes at most (both: 512 anchors a warp)
+static_assert(SORT_CAP_BIG >= GMF_MAX_READ_ANCHORS, "a read's anchors fit the large block");
+
+template <int T>
+struct SortSmem {
+    unsigned short hist[T / 32][256];
+    unsigned bin[256];
+    unsigned red[T / 32];
+    unsigned red2[T / 32];
+};
+
+template <int T, int CAP>
+constexpr size_t sort_smem_size() {
+    return (size_t)CAP * 8 + sizeof(SortSmem<T>);
+}
+
+// One stable pass by bits [shift, shift + 8) of key[]: src -> dst.
+template <int T>
+__device__ __forceinline__ void radix_pass(SortSmem<T>& S, const unsigned* key, const unsigned short* src,
+                                           unsigned short* dst, int n, int shift) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int rows = (n + T - 1) / T;  // per warp
+    const int first = w * rows * 32;
+    unsigned short* h = S.hist[w];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) reinterpret_cast<unsigned*>(h)[lane + 32 * x] = 0u;
+    __syncwarp();
+    unsigned at[SORT_ROWS];  // digit and place among the warp's anchors of that digit
+#pragma unroll
+    for (int i = 0; i < SORT_ROWS; ++i) {
+        at[i] = 0u;
+        if (i < rows) {
+            const int x = first + 32 * i + lane;
+            const unsigned d = x < n ? (key[src[x]] >> shift) & 255u : 256u;
+            const unsigned same = __match_any_sync(FULL_MASK, d);
+            const unsigned rank = __popc(same & lt);
+            unsigned base = 0;
+            if (x < n) base = h[d];
+            __syncwarp();
+            if (x < n && rank == 0) h[d] = (unsigned short)(base + __popc(same));
+            __syncwarp();
+            at[i] = d << 16 | (base + rank);
+        }
+    }
+    __syncthreads();
+    // offsets: digit by digit, within a digit warp by warp
+    if (tid < 256) {
+        unsigned run = 0;
+#pragma unroll 8
+        for (int v = 0; v < T / 32; ++v) {
+            const unsigned c = S.hist[v][tid];
+            S.hist[v][tid] = (unsigned short)run;
+            run += c;
+        }
+        unsigned incl = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(FULL_MASK, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) S.red[w] = incl;
+        S.bin[tid] = incl - run;
+    }
+    __syncthreads();
+    if (tid < 256) {
+        unsigned before = 0;
+        for (int v = 0; v < w; ++v) before += S.red[v];
+        S.bin[tid] += before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < SORT_ROWS; ++i) {
+        const int x = first + 32 * i + lane;
+        if (i < rows && x < n) {
+            const unsigned d = at[i] >> 16;
+            dst[S.bin[d] + h[d] + (at[i] & 0xFFFFu)] = src[x];
+        }
+    }
+    __syncthreads();
+}
+
+template <int T>
+__device__ __forceinline__ unsigned block_max(SortSmem<T>& S, unsigned v, unsigned* red) {
+    v = __reduce_max_sync(FULL_MASK, v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[0];
+    for (int w = 1; w < T / 32; ++w) v = max(v, red[w]);
+    return v;
+}
+
+__device__ __forceinline__ unsigned bits_of(unsigned v) { return 32u - __clz(v); }
+
+template <int T>
+__device__ void sort_read(const SortArgs& a, int r, int n, unsigned* key, unsigned short* ia, unsigned short* ib,
+                          SortSmem<T>& S, int* cnt) {
+    const int tid = threadIdx.x;
+    const int64_t a0 = a.read_off[r];
+    const int32_t* rp = a.read_pos + a0;
+    const int32_t* fp = a.ref_pos + a0;
+    const int32_t* ln = a.length + a0;
+    const int8_t* sd = a.strand + a0;
+    auto group = [&](int x) { return sd[x] == 1 ? 0u : (sd[x] == -1 ? 1u : 2u); };
+    auto read_end = [&](int x) { return (unsigned)(rp[x] + ln[x]) & 0x7fffffffu; };
+    if (tid < 3) cnt[tid] = 0;
+    __syncthreads();
+    // extremes, strand counts, and whether the anchors come in (strand, read_end) order
+    unsigned hi = 0, lo_c = 0, re_max = 0, c0 = 0, c1 = 0;  // lo_c: complement of the smallest
+    bool unordered = false;
+    for (int x = tid; x < n; x += T) {
+        const unsigned fe = (unsigned)(fp[x] + ln[x]) & 0x7fffffffu, re = read_end(x), g = group(x);
+        key[x] = fe;
+        ia[x] = (unsigned short)x;
+        hi = max(hi, fe);
+        lo_c = max(lo_c, ~fe);
+        re_max = max(re_max, re);
+        c0 += g == 0u;
+        c1 += g == 1u;
+        if (x > 0) {
+            const unsigned gp = group(x - 1);
+            unordered |= gp > g || (gp == g && read_end(x - 1) > re);
+        }
+    }
+    c0 = __reduce_add_sync(FULL_MASK, c0);
+    c1 = __reduce_add_sync(FULL_MASK, c1);
+    if ((tid & 31) == 0) {
+        if (c0) atomicAdd(&cnt[0], (int)c0);
+        if (c1) atomicAdd(&cnt[1], (int)c1);
+    }
+    hi = block_max<T>(S, hi, S.red);
+    const unsigned lo = ~block_max<T>(S, lo_c, S.red2);
+    unordered = __syncthreads_or(unordered);
+    const int n0 = cnt[0], m = cnt[0] + cnt[1];
+    const bool mixed = n0 != n && cnt[1] != n;  // several strands
+    unsigned short *src = ia, *dst = ib;
+    auto passes = [&](int bits) {
+        for (int b = 0; b < bits; b += 8) {
+            radix_pass<T>(S, key, src, dst, n, b);
+            unsigned short* t = src;
+            src = dst;
+            dst = t;
+        }
+    };
+    if (unordered) {
+        re_max = block_max<T>(S, re_max, S.red);
+        __syncthreads();
+        for (int x = tid; x < n; x += T) key[x] = read_end(x);
+        __syncthreads();
+        passes((int)bits_of(re_max));
+    }
+    const int nb = (int)bits_of(hi - lo);
+    const bool fold = mixed && nb <= 30;
+    __syncthreads();
+    for (int x = tid; x < n; x += T)
+        key[x] = (((unsigned)(fp[x] + ln[x]) & 0x7fffffffu) - lo) | (fold ? group(x) << nb : 0u);
+    __syncthreads();
+    passes(nb + (fold ? 2 : 0));
+    if (mixed && !fold) {
+        for (int x = tid; x < n; x += T) key[x] = group(x);
+        __syncthreads();
+        passes(2);
+    }
+    for (int x = tid; x < m; x += T) {
+        const int id = src[x];
+        a.perm[a0 + x] = id;
+        if (a.len_s) a.len_s[a0 + x] = ln[id];
+        a.ref_end_s[a0 + x] = (int32_t)((unsigned)(fp[id] + ln[id]) & 0x7fffffffu);
+        a.read_end_s[a0 + x] = (int32_t)read_end(id);
+    }
+    if (tid == 0) {
+        a.n_plus[r] = n0;
+        a.n_minus[r] = m - n0;
+    }
+}
+
+// Anchors of read r, or -1 (with the error noted) when the read cannot be
+// sorted: too many anchors for one read, or beyond what the workspace holds.
+// Such a read gets no sorted anchors (so no chains).
+__device__ __forceinline__ int sort_count(const SortArgs& a, int r, int* error) {
     const int64_t a0 = a.read_off[r];
     const int n = (int)(a.read_off[r + 1] - a0);
-    __shared__ int cnt[2];
-    if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
-    if (n > GMF_MAX_READ_ANCHORS || (a.cap >= 0 && a.read_off[r + 1] > a.cap)) {
-        // too many anchors for one read, or beyond what the workspace holds:
-        // the read gets no sorted anchors (so no chains) and the error word says why
+    *error = 0;
+    if (n > GMF_MAX_READ_ANCHORS) *error = 1;
+    else if (a.cap >= 0 && a.read_off[r + 1] > a.cap) *error = 4;
+    else if (n > SORT_CAP && 2 * a0 + next_pow2(n) > 2 * a.key_cap) *error = 2;
+    return *error ? -1 : n;
+}
+
+__global__ void __launch_bounds__(256) chain_sort_kernel(SortArgs a) {
+    extern __shared__ unsigned sort_smem[];
+    __shared__ int cnt[3];
+    const int r = blockIdx.x;
+    int error;
+    const int n = sort_count(a, r, &error);
+    if (n < 0) {
         if (threadIdx.x == 0) {
             a.n_plus[r] = 0;
             a.n_minus[r] = 0;
-            if (a.err) atomicOr(a.err, n > GMF_MAX_READ_ANCHORS ? 1 : 4);
+            if (a.err) atomicOr(a.err, error);
         }
         return;
     }
-    const int np2 = next_pow2(n > 0 ? n : 1);
-    unsigned long long* key;
-    int* idx;
-    if (np2 <= a.smem_elems) {
-        key = sm_keys;
-        idx = reinterpret_cast<int*>(sm_keys + a.smem_elems);
-    } else if (a.gkey && a.gidx && 2 * a0 + np2 <= 2 * a.key_cap) {
-        key = a.gkey + 2 * a0;
-        idx = a.gidx + 2 * a0;
-    } else {
-        if (threadIdx.x == 0) {
-            a.n_plus[r] = 0;
-            a.n_minus[r] = 0;
-            if (a.err) atomicOr(a.err, 2);
+    if (n > SORT_CAP) return;  // chain_sort_big_kernel
+    unsigned short* ia = reinterpret_cast<unsigned short*>(sort_smem + SORT_CAP);
+    sort_read<256>(a, r, n, sort_smem, ia, ia + SORT_CAP,
+                   *reinterpret_cast<SortSmem<256>*>(ia + 2 * SORT_CAP), cnt);
+}
+
+// Reads of more than SORT_CAP anchors: a block looks through every gridDim-th
+// read and sorts the large ones.
+__global__ void __launch_bounds__(1024) chain_sort_big_kernel(SortArgs a) {
+    extern __shared__ unsigned sort_smem[];
+    __shared__ int cnt[3];
+    __shared__ int n_found, found[1024];
+    unsigned short* ia = reinterpret_cast<unsigned short*>(sort_smem + SORT_CAP_BIG);
+    SortSmem<1024>& S = *reinterpret_cast<SortSmem<1024>*>(ia + 2 * SORT_CAP_BIG);
+    for (int64_t first = blockIdx.x; first < a.n_reads; first += (int64_t)gridDim.x * 1024) {
+        if (threadIdx.x == 0) n_found = 0;
+        __syncthreads();
+        const int64_t r = first + (int64_t)threadIdx.x * gridDim.x;
+        int error;
+        if (r < a.n_reads && sort_count(a, (int)r, &error) > SORT_CAP) found[atomicAdd(&n_found, 1)] = (int)r;
+        __syncthreads();
+        for (int k = 0; k < n_found; ++k) {
+            const int q = found[k];
+            sort_read<1024>(a, q, (int)(a.read_off[q + 1] - a.read_off[q]), sort_smem, ia, ia + SORT_CAP_BIG, S, cnt);
+            __syncthreads();
         }
-        return;
-    }
-    __syncthreads();
-    for (int x = threadIdx.x; x < np2; x += blockDim.x) {
-        unsigned long long k = ~0ull;
-        int ix = 0x7fffffff;
-        if (x < n) {
-            const int8_t s = a.strand[a0 + x];
-            const unsigned long long grp = s == 1 ? 0ull : (s == -1 ? 1ull : 2ull);
-            const unsigned re = (unsigned)(a.read_pos[a0 + x] + a.length[a0 + x]);
-            const unsigned fe = (unsigned)(a.ref_pos[a0 + x] + a.length[a0 + x]);
-            k = (grp << 62) | ((unsigned long long)(fe & 0x7fffffffu) << 31) |
-                (unsigned long long)(re & 0x7fffffffu);
-            ix = x;
-            if (grp < 2) atomicAdd(&cnt[grp], 1);
-        }
-        key[x] = k;
-        idx[x] = ix;
-    }
-    __syncthreads();
-    // the shared-memory call is spelled out so the sort uses shared loads
-    if (np2 <= a.smem_elems)
-        block_bitonic(sm_keys, reinterpret_cast<int*>(sm_keys + a.smem_elems), np2);
-    else
-        block_bitonic(key, idx, np2);
-    const int m = cnt[0] + cnt[1];
-    for (int x = threadIdx.x; x < m; x += blockDim.x) {
-        const unsigned long long k = key[x];
-        a.perm[a0 + x] = idx[x];
-        if (a.len_s) a.len_s[a0 + x] = a.length[a0 + idx[x]];
-        a.ref_end_s[a0 + x] = (int32_t)((k >> 31) & 0x7fffffffu);
-        a.read_end_s[a0 + x] = (int32_t)(k & 0x7fffffffu);
-    }
-    if (threadIdx.x == 0) {
-        a.n_plus[r] = cnt[0];
-        a.n_minus[r] = cnt[1];
     }
 }
 
@@ -1099,18 +1273,16 @@ using namespace gmf;
 
 namespace {
 
-// Shared-memory sort buffers: 4096 keys (48 KB) for the per-read sort and
-// 2048 (24 KB) for the per-strand peel, so 4 and 8 CTAs fit an SM (the peel's
-// serial walk runs in 8 blocks of 4 warps per SM); larger reads / strands
-// sort in their own workspace range instead.  The peel buffer also holds a
-// strand's walk state (6 bytes per anchor) beside its sorted starts.
-int sort_smem_elems() { return 4096; }
+// Shared-memory sort buffer of the per-strand peel: 2048 keys (24 KB), so 8
+// CTAs fit an SM (the peel's serial walk runs in 8 blocks of 4 warps per SM);
+// larger strands sort in their own workspace range instead.  The buffer also
+// holds a strand's walk state (6 bytes per anchor) beside its sorted starts.
 int peel_smem_elems() { return 2048; }
 
 size_t sort_smem_bytes(int elems) { return (size_t)elems * (sizeof(unsigned long long) + sizeof(int)); }
 
-int launch_sort(const gmf_anchor_batch* an, const gmf_sorted_anchors* so, int32_t* len_s, unsigned long long* gkey,
-                int* gidx, int64_t cap, int64_t key_cap, int* err, cudaStream_t stream) {
+int launch_sort(const gmf_anchor_batch* an, const gmf_sorted_anchors* so, int32_t* len_s, int64_t cap,
+                int64_t key_cap, int* err, cudaStream_t stream) {
     SortArgs s;
     s.n_reads = an->n_reads;
     s.read_off = an->read_off;
@@ -1124,16 +1296,15 @@ int launch_sort(const gmf_anchor_batch* an, const gmf_sorted_anchors* so, int32_
     s.read_end_s = so->read_end;
     s.ref_end_s = so->ref_end;
     s.len_s = len_s;
-    s.gkey = gkey;
-    s.gidx = gidx;
-    s.smem_elems = sort_smem_elems();
     s.cap = cap;
     s.key_cap = key_cap;
     s.err = err;
-    const size_t smem = sort_smem_bytes(s.smem_elems);
-    GMF_CUDA_TRY(cudaFuncSetAttribute(chain_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-    chain_sort_kernel<<<an->n_reads, 256, smem, stream>>>(s);
+    constexpr size_t small = sort_smem_size<256, SORT_CAP>(), big = sort_smem_size<1024, SORT_CAP_BIG>();
+    GMF_CUDA_TRY(cudaFuncSetAttribute(chain_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small));
+    chain_sort_kernel<<<an->n_reads, 256, small, stream>>>(s);
+    GMF_CUDA_TRY(cudaGetLastError());
+    GMF_CUDA_TRY(cudaFuncSetAttribute(chain_sort_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)big));
+    chain_sort_big_kernel<<<std::min(an->n_reads, 148), 1024, big, stream>>>(s);
     return cuda_status(cudaGetLastError());
 }
 
@@ -1242,19 +1413,14 @@ extern "C" int gmf_chain_sort(const gmf_anchor_batch* an, const gmf_sorted_ancho
         return GMF_ERR_INVALID_ARGUMENT;
     if (!workspace || workspace_bytes < 256) return GMF_ERR_WORKSPACE;
     GMF_BIND_STREAM(stream);
-    // reads too large for shared memory sort in 12 * 2 bytes per anchor of
-    // workspace (gmf_chain_workspace_bytes covers it)
+    // reads of more than SORT_CAP anchors are sorted when the workspace has 12 * 2 bytes per anchor up to
+    // theirs (gmf_chain_workspace_bytes covers it)
     const size_t A = (workspace_bytes - 256) / 24;
     char* p = (char*)workspace;
     int* err = (int*)p;
-    unsigned long long* gkey = (unsigned long long*)(p + 256);
-    int* gidx = (int*)(p + 256 + align256(2 * A * 8));
-    if (256 + align256(2 * A * 8) + 2 * A * 4 > workspace_bytes) {
-        gidx = nullptr;
-        gkey = nullptr;
-    }
+    const bool fits = 256 + align256(2 * A * 8) + 2 * A * 4 <= workspace_bytes;
     GMF_CUDA_TRY(cudaMemsetAsync(err, 0, 4, (cudaStream_t)stream));
-    return launch_sort(an, so, nullptr, gkey, gidx, -1, (int64_t)A, err, (cudaStream_t)stream);
+    return launch_sort(an, so, nullptr, -1, fits ? (int64_t)A : 0, err, (cudaStream_t)stream);
 }
 
 extern "C" size_t gmf_chain_workspace_bytes(int32_t n_reads, int64_t n_anchors) {
@@ -1343,7 +1509,7 @@ extern "C" int gmf_chain_batch(const gmf_anchor_batch* an, const gmf_chain_param
     GMF_CUDA_TRY(cudaMemsetAsync(err, 0, 256, stream));
     int st;
     if (!sorted_in) {
-        st = launch_sort(an, &so, mem_tmp, gkey, gidx, (int64_t)A, (int64_t)A, err, stream);
+        st = launch_sort(an, &so, mem_tmp, (int64_t)A, (int64_t)A, err, stream);
         if (st) return st;
     }
     DpArgs d{};

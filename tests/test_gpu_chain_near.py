@@ -65,3 +65,30 @@ def test_selection_cutoffs_match_oracle_in_a_large_batch(kw):
     from graphmambaformer_b200.config import ChainingConfig
 
     _check(_dense_batch(5, 900, copies=75), ChainingConfig(max_lookback=50, max_gap=300, **kw))
+
+
+@pytest.mark.parametrize("top,shuffle", [(60, True), (3000, False), (200_000, True), (2**31 - 100, True),
+                                         (2**31 - 100, False), (2**30 - 40, True)])
+def test_sorting_any_order_strand_and_size(top, shuffle):
+    """Anchors in read order per strand (as seeding writes them) and in any
+    order, strands interleaved and strands that take no part, many equal
+    keys, coordinates up to 31 bits, and read sizes around the sort's block
+    sizes."""
+    from graphmambaformer_b200.chaining import AnchorCSR
+    from graphmambaformer_b200.config import ChainingConfig
+
+    rng = np.random.default_rng(top % 1000 + shuffle)
+    counts = [0, 1, 2, 31, 32, 33, 255, 256, 257, 511, 513, 4095, 4096, 4097, 8200, 16384, 700, 0, 5]
+    off = np.zeros(len(counts) + 1, np.int64)
+    np.cumsum(counts, out=off[1:])
+    n = int(off[-1])
+    t = rng.integers(0, top, n)
+    q = np.minimum(np.where(rng.random(n) < 0.5, t % 20_000, rng.integers(0, 20_000, n)), top)
+    length = np.full(n, 15)
+    strand = rng.choice([1, -1, 0, 2], n, p=[0.5, 0.4, 0.05, 0.05]).astype(np.int8)
+    if not shuffle:
+        for a, b in zip(off[:-1], off[1:]):
+            o = np.lexsort((q[a:b], -strand[a:b].astype(int)))
+            q[a:b], t[a:b], strand[a:b] = q[a:b][o], t[a:b][o], strand[a:b][o]
+    batch = AnchorCSR(off, q.astype(np.int32), t.astype(np.int32), length.astype(np.int32), strand)
+    _check(batch, ChainingConfig(max_lookback=20, max_gap=2000))
