@@ -286,6 +286,8 @@ _SIGNATURES = {
     "gmf_wfa_distance": (c_int, [POINTER(GmfWfaPairs), c_int32, c_void_p, c_void_p, c_size_t, c_void_p]),
     "gmf_wfa_align": (c_int, [POINTER(GmfWfaPairs), c_void_p, c_int32, POINTER(GmfWfaResults), c_void_p,
                               c_size_t, c_void_p]),
+    "gmf_wfa_align_direct": (c_int, [POINTER(GmfWfaPairs), c_int32, c_void_p, POINTER(GmfWfaResults), c_void_p,
+                                     c_size_t, c_void_p]),
 }
 
 _lib = None

@@ -8,12 +8,12 @@ Drop-in for the reference's wavefront pieces:
 * :func:`wfa_distance` -- ``accel/cuda_kernels.py`` L569-600 (padded
   ``(B, L)`` code tensors in, int32 distances out, ``-1`` beyond the bound).
 
-A batch runs in two device passes: ``gmf_wfa_distance`` finds every pair's
-distance (one warp per pair, the live wavefronts in shared memory), then
-``gmf_wfa_align`` recomputes each pair's wavefronts to exactly that distance,
-keeping the history ((d+1)^2 offsets, carved from the workspace), and walks
-it back to the CIGAR with the reference's tie order.  Pairs whose histories
-together exceed the budget are split over several calls.  Every computation
+A batch runs in one device pass: ``gmf_wfa_align_direct`` finds every pair's
+distance with its wavefronts kept in the workspace as it goes, and walks them
+back to the CIGAR with the reference's tie order.  Pairs whose wavefronts did
+not fit the workspace are replayed to their known distance by
+``gmf_wfa_align`` ((d+1)^2 offsets each), split over several calls where they
+exceed the budget.  Every computation
 runs in the gmf CUDA library; without a GPU the calls raise.
 """
 
@@ -323,50 +323,85 @@ def align_device_pairs(dp: DeviceWfaPairs, max_distance: int = 4096, stream: Opt
         return _align_device(dp, max_distance, stream, sp, traceback, history_budget, workspace)
 
 
+def direct_entries(qlen: np.ndarray, tlen: np.ndarray, max_distance: int) -> int:
+    """History entries that hold the chunks of pairs with up to about 8%
+    differences (see gmf_wfa_align_direct)."""
+    longest = np.maximum(qlen, tlen).astype(np.int64)
+    d = np.minimum(np.minimum(longest, max_distance), longest * 8 // 100 + 48)
+    c = d // 32 + 1
+    return int((1024 * c * c + 2 * c).sum())
+
+
 def _align_device(dp, max_distance, stream, sp, traceback, history_budget, workspace) -> WfaResult:
-    dist_d = wfa_distances(dp, max_distance, stream, workspace=workspace)
-    h_dist = dist_d.to("cpu", non_blocking=True)
-    stream.synchronize()
-    h_dist = h_dist.numpy().copy()
+    dev, n = dp.device, dp.n
     if not traceback:
-        return WfaResult(h_dist)
-    counts = np.zeros((dp.n, 4), np.int32)
-    cstart = np.zeros(dp.n, np.int64)
-    clen = np.full(dp.n, -1, np.int32)
-    words_all: list = []
-    base = 0
-    # chunks whose histories fit the budget (a pair above it alone)
-    hist = np.where((h_dist >= 0) & (dp.h_qlen > 0) & (dp.h_tlen > 0),
-                    (h_dist.astype(np.int64) + 1) ** 2, 0)
-    chunks = history_chunks(hist, history_budget)
-    for c0, c1 in chunks:
-        idx = np.arange(c0, c1, dtype=np.int64)
-        if len(chunks) == 1:
-            sub, d_sub, h_d = dp, dist_d, h_dist
-        else:
-            sub, d_sub, h_d = _sub_batch(dp, dist_d, h_dist, idx)
-        out = _run_align(sub, d_sub, h_d, sp, workspace)
-        host = {k: v.to("cpu", non_blocking=True) for k, v in out.items() if k != "cigar"}
+        h_dist = wfa_distances(dp, max_distance, stream, workspace=workspace).to("cpu", non_blocking=True)
         stream.synchronize()
-        if int(host["err"][0]) & _native.GMF_SWF_CAPACITY:
-            raise RuntimeError("gmf_wfa_align: CIGAR output capacity exhausted")
-        if int(host["err"][0]) & _native.GMF_SWF_WORKSPACE:
-            raise RuntimeError("gmf_wfa_align: history workspace exhausted")
-        if int(host["err"][0]) & _native.GMF_SWF_INTERNAL:
-            raise RuntimeError("gmf_wfa_align: a distance does not belong to its pair")
-        used = int(host["used"][0])
-        words = np.zeros(0, np.uint32)
-        if used:
-            hw = out["cigar"][:used].to("cpu", non_blocking=True)
+        return WfaResult(h_dist.numpy().copy())
+    md = _check_bound(max_distance, dp.max_len)
+    lib = _native.lib()
+    order = to_device(np.argsort(-(dp.h_qlen.astype(np.int64) + dp.h_tlen), kind="stable").astype(np.int32), dev)
+    need = int(lib.gmf_wfa_workspace_bytes(n, dp.max_len, md,
+                                           min(int(history_budget), direct_entries(dp.h_qlen, dp.h_tlen, md))))
+    ws = _ws(workspace, dev, need)
+    cap = int(dp.h_qlen.astype(np.int64).sum() + dp.h_tlen.astype(np.int64).sum() + n)
+    # one buffer for the fixed-size results: starts and the word count, then counts, lengths, distances, flags
+    fixed = torch.empty(2 * n + 2 + 6 * n + 1, dtype=torch.int32, device=dev)
+    cigar = torch.empty(max(cap, 1), dtype=torch.int32, device=dev)
+    p8 = fixed.data_ptr()
+    p4 = p8 + 8 * (n + 1)
+    res = _native.GmfWfaResults(p4, ptr(cigar), cigar.numel(), p8, p4 + 16 * n, p8 + 8 * n, p4 + 24 * n)
+    pairs = dp.c(order)
+    bind(dev, sp)
+    st = lib.gmf_wfa_align_direct(ctypes.byref(pairs), md, ctypes.c_void_p(p4 + 20 * n), ctypes.byref(res),
+                                  ctypes.c_void_p(ws.data_ptr()), need, ctypes.c_void_p(sp))
+    _native.check("gmf_wfa_align_direct", st)
+    host = fixed.to("cpu", non_blocking=True)
+    stream.synchronize()
+    host = host.numpy()
+    i64 = host[: 2 * (n + 1)].view(np.int64)
+    rest = host[2 * (n + 1):]
+    cstart, used = i64[:n].copy(), int(i64[n])
+    counts, clen, h_dist = rest[: 4 * n].reshape(n, 4).copy(), rest[4 * n: 5 * n].copy(), rest[5 * n: 6 * n].copy()
+    _check_flags(int(rest[6 * n]))
+    words_all = [_fetch_words(cigar, used, stream)]
+    base = used
+    # pairs whose wavefronts did not fit: replayed in chunks whose histories fit the budget (a pair above it alone)
+    left = np.nonzero(clen == -2)[0]
+    if len(left):
+        dist_d = to_device(h_dist, dev)
+        for c0, c1 in history_chunks((h_dist[left].astype(np.int64) + 1) ** 2, history_budget):
+            idx = left[c0:c1]
+            sub, d_sub, h_d = _sub_batch(dp, dist_d, h_dist, idx)
+            out = _run_align(sub, d_sub, h_d, sp, workspace)
+            part = {k: v.to("cpu", non_blocking=True) for k, v in out.items() if k != "cigar"}
             stream.synchronize()
-            words = hw.numpy().view(np.uint32).copy()
-        counts[idx] = host["counts"].numpy()
-        cstart[idx] = host["cstart"].numpy() + base
-        clen[idx] = host["clen"].numpy()
-        words_all.append(words)
-        base += used
-    words = np.concatenate(words_all) if words_all else np.zeros(0, np.uint32)
+            _check_flags(int(part["err"][0]))
+            used = int(part["used"][0])
+            words_all.append(_fetch_words(out["cigar"], used, stream))
+            counts[idx] = part["counts"].numpy()
+            cstart[idx] = part["cstart"].numpy() + base
+            clen[idx] = part["clen"].numpy()
+            base += used
+    words = np.concatenate(words_all) if len(words_all) > 1 else words_all[0]
     return WfaResult(h_dist, counts, words, cstart, clen)
+
+
+def _check_flags(flags: int) -> None:
+    if flags & _native.GMF_SWF_CAPACITY:
+        raise RuntimeError("gmf_wfa_align: CIGAR output capacity exhausted")
+    if flags & _native.GMF_SWF_WORKSPACE:
+        raise RuntimeError("gmf_wfa_align: history workspace exhausted")
+    if flags & _native.GMF_SWF_INTERNAL:
+        raise RuntimeError("gmf_wfa_align: a distance does not belong to its pair")
+
+
+def _fetch_words(cigar: torch.Tensor, used: int, stream) -> np.ndarray:
+    if not used:
+        return np.zeros(0, np.uint32)
+    hw = cigar[:used].to("cpu", non_blocking=True)
+    stream.synchronize()
+    return hw.numpy().view(np.uint32).copy()
 
 
 def wfa_distance(query: torch.Tensor, target: torch.Tensor, query_len: torch.Tensor, target_len: torch.Tensor,
