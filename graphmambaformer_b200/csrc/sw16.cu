@@ -336,7 +336,9 @@ struct CoopLinks {
 // chunk's values at hand.  Bounds of 95, 80 and 72 registers (20, 24 and 28
 // warps an SM instead of 16) ran the same pairs at 709, 656 and 551 GCUPS
 // (32 lanes) and a lone warp's steps 10, 31 and 35% slower, so the kernels ask
-// for 16 warps an SM.
+// for 16 warps an SM.  Pairs of 16 lanes, short and alike, take 20: their last
+// wave counts for more (2,000 / 10,000 / 20,000 pairs of 150 bp: 76 / 170 / 299
+// us with 16 warps, 70 / 162 / 308 us with 20).
 template <int L, int NW, bool TB, bool XD, int EM>
 __device__ __forceinline__ void sw16_rows(const SwArgs& a, const PairGeo& G, bool active, const Grp<L>& grp,
                                           const GroupSmem& sm, int w, int nstrips, int n_chunks, int last_chunk,
@@ -740,7 +742,7 @@ __device__ void sw16_group(const SwArgs& a, int p, const Grp<L>& grp, const Grou
 // one, and to different schedulers of the SM in the blocks of later waves, so
 // a short list spreads over the SMs instead of filling the first blocks.
 template <int L, bool TB, bool XD, int EM>
-__global__ void __launch_bounds__(128, 4) sw16_kernel(SwArgs a) {
+__global__ void __launch_bounds__(128, L == 16 ? 5 : 4) sw16_kernel(SwArgs a) {
     extern __shared__ uint4 sw16_smem[];
     constexpr int GPW = 32 / L;  // pairs per warp
     constexpr int CLS = L == 8 ? CLS_I16_L8 : (L == 16 ? CLS_I16_L16 : CLS_I16_L32);

@@ -31,9 +31,9 @@
 // What bounds it is the critical path: a 20 kb ONT-like pair takes ~1,000
 // wavefronts one after another, whatever else the GPU does.  So a long pair's
 // block has 1,024 threads (a wavefront of 2s+1 diagonals in few turns), a turn
-// compares 4 or 8 codes at once with 32-bit word indices, and the history is kept while the distance is found (in chunks of 32 wavefronts,
-// allocated as the pair goes) instead of replaying every pair to its known
-// distance.  Measured on one B200, 4,000 mixed pairs of 150-20,000 bases:
+// compares 4 or 8 codes at once with 32-bit word indices, and the history is
+// kept while the distance is found (in chunks of 32 wavefronts, allocated as
+// the pair goes) instead of replaying every pair to its known distance.  Measured on one B200, 4,000 mixed pairs of 150-20,000 bases:
 // forward 3,711 + 4,061 us (distance, then replay with history) -> 1,654 us,
 // walk 1,091 -> 281 us.
 
