@@ -72,5 +72,25 @@ def to_device(a: np.ndarray, device: torch.device, stream=None, pinned: bool = T
     return t.to(device, non_blocking=True)
 
 
+def packed_layout(nbytes) -> tuple:
+    """Byte offsets of arrays laid one after another on 256-byte boundaries
+    (every kernel's widest access), and the total."""
+    off, n = [], 0
+    for b in nbytes:
+        off.append(n)
+        n += -(-int(b) // 256) * 256
+    return off, max(n, 256)
+
+
+def pack_host(arrays, off, host: torch.Tensor) -> None:
+    """Write the arrays at their offsets of a host byte buffer."""
+    flat = host.numpy()
+    for a, o in zip(arrays, off):
+        if a.nbytes >= 1 << 20:  # torch's host copy runs on several threads
+            host[o: o + a.nbytes].copy_(torch.from_numpy(a.reshape(-1).view(np.uint8)))
+        elif a.nbytes:
+            flat[o: o + a.nbytes].view(a.dtype)[...] = a.reshape(-1)
+
+
 def np_ptr(a: np.ndarray) -> ctypes.c_void_p:
     return a.ctypes.data_as(ctypes.c_void_p)

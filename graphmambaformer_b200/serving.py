@@ -41,9 +41,16 @@ import torch
 from . import _native
 from .chaining import LUTS, AnchorCSR, ChainingConfig, chain_params
 from .config import ExtensionConfig
-from .device import bind, require_cuda
+from .device import bind, pack_host, packed_layout, require_cuda
 from .extension import longest_first, params_from_config
 from .session import _Buffers
+
+
+# A batch's CIGAR words come back beside its other results when the buffer
+# they lie in is at most this many bytes: that much more to copy takes about
+# 5 us, a second wait for the stream about 15.  A larger buffer waits for the
+# count of words used.
+CIGAR_WITH_RESULTS = 256 << 10
 
 
 def estimate_bytes(read_lens: np.ndarray, n_anchors: int, cfg: ExtensionConfig, max_chains: int) -> int:
@@ -118,6 +125,17 @@ class BatchAlignments:
             yield self[i]
 
 
+def _join_codes(reads, out: np.ndarray, total: int) -> None:
+    """The reads' codes, one after another, in ``out`` (one zero when there are none)."""
+    if total == 0:
+        out[:] = 0
+        return
+    try:
+        np.concatenate(reads, out=out, casting="no")
+    except (TypeError, ValueError):  # not int8 arrays: converted as a whole
+        out[:] = np.concatenate(reads).astype(np.int8)
+
+
 class BatchAligner:
     """The device pipeline for one batch of reads on one stream (grow-only
     buffers, reused between batches)."""
@@ -149,60 +167,61 @@ class BatchAligner:
             return []
         if anchors is None and self.index is None:
             raise ValueError("anchors are required unless the aligner holds a minimizer index")
-        s, up, db = self.stream, self.buf.upload, self.buf.device_buf
+        s, db = self.stream, self.buf.device_buf
         sp = int(s.cuda_stream)
         bind(self.device, sp)
         rl = np.array([len(x) for x in reads], np.int64)
         roff = np.zeros(R + 1, np.int64)
         np.cumsum(rl, out=roff[1:])
-        codes = np.concatenate(reads).astype(np.int8) if roff[-1] else np.zeros(1, np.int8)
-        reads_d = up("reads", codes, s)
-        pad = lambda x, dt: x if len(x) else np.zeros(1, dt)  # noqa: E731
-        if anchors is None:  # device seeding: both orientations, forward anchors first
-            sd = self.index.seed_device(reads_d[: len(codes)], up("roff", roff, s), R, True, stream=s)
-            ro, rp, fp, ln, st = sd["read_off"], sd["read_pos"], sd["ref_pos"], sd["length"], sd["strand"]
+        a = None if anchors is None else AnchorCSR.of(anchors)
+        if a is not None and R != len(a):
+            raise ValueError("one anchor set per read is required")
+        # the batch's inputs in one copy: offsets or anchors, then the reads joined in place
+        cols = [roff] if a is None else [np.ascontiguousarray(x) for x in
+                                         (a.read_off, a.read_pos, a.ref_pos, a.length, a.strand)]
+        n_codes = max(int(roff[-1]), 1)
+        at, nb = packed_layout([x.nbytes for x in cols] + [n_codes])
+        h_in, d_in = self.buf.packed("in", nb)
+        pack_host(cols, at, h_in)
+        _join_codes(reads, h_in.numpy()[at[-1]: at[-1] + n_codes].view(np.int8), int(roff[-1]))
+        with torch.cuda.stream(s):
+            d_in[:nb].copy_(h_in[:nb], non_blocking=True)
+        reads_d = d_in[at[-1]: at[-1] + n_codes].view(torch.int8)
+        if a is None:  # device seeding: both orientations, forward anchors first
+            sd = self.index.seed_device(reads_d, d_in[: roff.nbytes].view(torch.int64), R, True, stream=s)
+            ro, rp, fp, ln, st = (sd[x].data_ptr() for x in ("read_off", "read_pos", "ref_pos", "length", "strand"))
             A = int(sd["n_anchors"])
             per_read = int(sd["max_read_anchors"])
         else:
-            a = AnchorCSR.of(anchors)
-            if R != len(a):
-                raise ValueError("one anchor set per read is required")
             A = int(a.read_off[-1])
             per_read = int(np.diff(a.read_off).max(initial=0))
-            ro = up("ro", a.read_off, s)
-            rp = up("rp", pad(a.read_pos, np.int32), s)
-            fp = up("fp", pad(a.ref_pos, np.int32), s)
-            ln = up("ln", pad(a.length, np.int32), s)
-            st = up("st", pad(a.strand, np.int8), s)
+            ro, rp, fp, ln, st = (d_in.data_ptr() + x for x in at[:5])
         if per_read > _native.MAX_READ_ANCHORS:
             raise ValueError(f"a read has more than {_native.MAX_READ_ANCHORS} anchors")
         mc = self.cp.max_chains
-        o = dict(n=db("n", R, torch.int32), score=db("score", R * mc, torch.float64),
-                 strand=db("strand", R * mc, torch.int32), span=db("span", 4 * R * mc, torch.int32),
-                 prim=db("prim", R * mc, torch.int32), nmem=db("nmem", R * mc, torch.int32),
-                 mem=db("mem", max(A, 1), torch.int32))
+        # the chain records that come back lie side by side, for one copy
+        rec = (("n", R, np.int32), ("strand", R * mc, np.int32), ("spread", R * mc, np.int32),
+               ("prim", R * mc, np.int32), ("span", 4 * R * mc, np.int32), ("score", R * mc, np.float64))
+        rat, rnb = packed_layout([n * np.dtype(dt).itemsize for _, n, dt in rec])
+        h_rec, d_rec = self.buf.packed("chains", rnb)
+        o = {k: d_rec.data_ptr() + x for (k, _, _), x in zip(rec, rat)}
+        nmem, mem = db("nmem", R * mc, torch.int32), db("mem", max(A, 1), torch.int32)
         need = int(_native.lib().gmf_chain_workspace_bytes(R, A))
         ws = db("cws", need, torch.uint8)
-        batch_c = _native.GmfAnchorBatch(R, ro.data_ptr(), rp.data_ptr(), fp.data_ptr(), ln.data_ptr(), st.data_ptr())
-        res_c = _native.GmfChainResults(o["n"].data_ptr(), o["score"].data_ptr(), o["strand"].data_ptr(),
-                                        o["span"].data_ptr(), o["prim"].data_ptr(), o["nmem"].data_ptr(),
-                                        o["mem"].data_ptr())
+        batch_c = _native.GmfAnchorBatch(R, ro, rp, fp, ln, st)
+        res_c = _native.GmfChainResults(o["n"], o["score"], o["strand"], o["span"], o["prim"], nmem.data_ptr(),
+                                        mem.data_ptr())
         self._call("gmf_chain_batch", ctypes.byref(batch_c), ctypes.byref(self.cp),
                    ctypes.c_void_p(self.lut.data_ptr()), self.lut.numel(), None, None, None, ctypes.byref(res_c),
                    ctypes.c_void_p(ws.data_ptr()), need, ctypes.c_void_p(sp))
         # the diagonal spread of every chain, on the device beside the chain records
-        spread_d = db("spread", R * mc, torch.int32)
         self._call("gmf_chain_spread", ctypes.byref(batch_c), ctypes.byref(res_c), mc,
-                   ctypes.c_void_p(spread_d.data_ptr()), ctypes.c_void_p(sp))
-        dl = self.buf.download
-        h = {k: dl("h_" + k, t, n, s) for k, t, n in
-             (("n", o["n"], R), ("strand", o["strand"], R * mc), ("span", o["span"], 4 * R * mc),
-              ("spread", spread_d, R * mc), ("score", o["score"], R * mc), ("prim", o["prim"], R * mc))}
+                   ctypes.c_void_p(o["spread"]), ctypes.c_void_p(sp))
+        h = self._download(h_rec, d_rec, rnb, rec, rat)
         s.synchronize()
-        n_ch = np.minimum(h["n"][:R].numpy(), mc)
-        strand = h["strand"][: R * mc].numpy().reshape(R, mc)
-        span = h["span"][: 4 * R * mc].numpy().reshape(R, mc, 4)
-        spread_all = h["spread"][: R * mc].numpy().reshape(R, mc)
+        n_ch = np.minimum(h["n"], mc)
+        strand, spread_all = h["strand"].reshape(R, mc), h["spread"].reshape(R, mc)
+        span = h["span"].reshape(R, mc, 4)
 
         # ---- one pair per kept chain, in read order ----
         cr, ck = np.nonzero(np.arange(mc)[None, :] < n_ch[:, None])  # (read, slot) of every chain
@@ -212,8 +231,8 @@ class BatchAligner:
         if C == 0:
             return BatchAlignments.empty(R)
         spread = spread_all[cr, ck].astype(np.int64)
-        chains = dict(score=h["score"][: R * mc].numpy().reshape(R, mc)[cr, ck],
-                      strand=strand[cr, ck].copy(), prim=h["prim"][: R * mc].numpy().reshape(R, mc)[cr, ck])
+        chains = dict(score=h["score"].reshape(R, mc)[cr, ck], strand=strand[cr, ck],
+                      prim=h["prim"].reshape(R, mc)[cr, ck])
         rc = strand[cr, ck] < 0
         sp4 = span[cr, ck].astype(np.int64)  # read_start, read_end, ref_start, ref_end
         if self.ecfg.algorithm == "wfa":
@@ -222,11 +241,21 @@ class BatchAligner:
         cols, words = self._extend_sw(R, rl, roff, reads_d, cr, rc, sp4, spread, shared=True)
         return BatchAlignments(R, chain_off, cols, words, chains=chains)
 
-    def _gather(self, tag: str, reads_d, roff, rl, cr, rc, wstart, wlen) -> tuple:
+    def _download(self, host, dev, nbytes: int, cols, at) -> dict:
+        """Copy packed results to the host (valid once the stream is waited
+        for): the columns (name, count, type) as arrays on the pinned bytes,
+        which the next batch reuses."""
+        with torch.cuda.stream(self.stream):
+            host[:nbytes].copy_(dev[:nbytes], non_blocking=True)
+        flat = host.numpy()
+        return {k: flat[x: x + n * np.dtype(dt).itemsize].view(dt) for (k, n, dt), x in zip(cols, at)}
+
+    def _gather(self, tag: str, reads_d, roff, rl, cr, rc, wstart, wlen, more=()) -> tuple:
         """Queries (reverse-complemented for strand -1) and reference
-        windows of the pairs, gathered from the resident buffers."""
-        s, up, db = self.stream, self.buf.upload, self.buf.device_buf
-        sp = int(s.cuda_stream)
+        windows of the pairs, gathered from the resident buffers.  Columns
+        in ``more`` go up in the same copy; their addresses come last."""
+        s, db = self.stream, self.buf.device_buf
+        vp, sp = ctypes.c_void_p, int(s.cuda_stream)
         C = len(cr)
         rlen = rl[cr]
         qoff = np.zeros(C + 1, np.int64)
@@ -235,24 +264,22 @@ class BatchAligner:
         np.cumsum(wlen, out=toff[1:])
         qd = db(tag + "q", max(int(qoff[-1]), 1), torch.int8)
         td = db(tag + "t", max(int(toff[-1]), 1), torch.int8)
-        qs_d, ql_d = up(tag + "qs", roff[cr], s), up(tag + "ql", rlen.astype(np.int32), s)
-        rc_d, qo_d = up(tag + "rc", rc.astype(np.int8), s), up(tag + "qo", qoff, s)
-        ts_d, tl_d, to_d = up(tag + "ts", wstart, s), up(tag + "tl", wlen.astype(np.int32), s), up(tag + "to", toff, s)
-        self._call("gmf_gather_segments", ctypes.c_void_p(reads_d.data_ptr()), int(roff[-1]), C,
-                   ctypes.c_void_p(qs_d.data_ptr()), ctypes.c_void_p(ql_d.data_ptr()),
-                   ctypes.c_void_p(rc_d.data_ptr()), ctypes.c_void_p(qd.data_ptr()),
-                   ctypes.c_void_p(qo_d.data_ptr()), ctypes.c_void_p(sp))
-        self._call("gmf_gather_segments", ctypes.c_void_p(self.ref_d.data_ptr()), self.ref_len, C,
-                   ctypes.c_void_p(ts_d.data_ptr()), ctypes.c_void_p(tl_d.data_ptr()), None,
-                   ctypes.c_void_p(td.data_ptr()), ctypes.c_void_p(to_d.data_ptr()), ctypes.c_void_p(sp))
-        return qd, qo_d, td, to_d, qoff, toff
+        cols = [qoff, toff, roff[cr], wstart, rlen.astype(np.int32), wlen.astype(np.int32), rc.astype(np.int8), *more]
+        up, at = self.buf.upload_packed(tag + "cols", cols, s)
+        qo, to, qs, ts, ql, tl, rcp, *rest = (up.data_ptr() + x for x in at)
+        self._call("gmf_gather_segments", vp(reads_d.data_ptr()), int(roff[-1]), C, vp(qs), vp(ql), vp(rcp),
+                   vp(qd.data_ptr()), vp(qo), vp(sp))
+        self._call("gmf_gather_segments", vp(self.ref_d.data_ptr()), self.ref_len, C, vp(ts), vp(tl), None,
+                   vp(td.data_ptr()), vp(to), vp(sp))
+        qo_d, to_d = (up[x: x + 8 * (C + 1)].view(torch.int64) for x in at[:2])
+        return qd, qo_d, td, to_d, qoff, toff, rest
 
     def _extend_sw(self, R, rl, roff, reads_d, cr, rc, sp4, spread, shared: bool) -> list:
         """Banded SW + traceback of the pairs (extension.py L489-641).  With
         ``shared``, the chains of a read take its widest band and stop
         together under x-drop, as one extend_chains call; without, every
         chain is a call of its own (the WFA fallback)."""
-        s, up, db, dl = self.stream, self.buf.upload, self.buf.device_buf, self.buf.download
+        s, db = self.stream, self.buf.device_buf
         sp = int(s.cuda_stream)
         cfg = self.ecfg
         C = len(cr)
@@ -272,48 +299,45 @@ class BatchAligner:
             np.cumsum(np.bincount(cr, minlength=R), out=goff[1:])
         hb = hb.astype(np.int32)
         boff = (diag - wstart).astype(np.int32)
-        qd, qo_d, td, to_d, qoff, toff = self._gather("s", reads_d, roff, rl, cr, rc, wstart, wlen)
-        hb_d, bo_d = up("hb", hb, s), up("bo", boff, s)
-        ord_d = up("ord", longest_first(rlen.astype(np.int32), hb), s)
-        out = dict(score=db("sc", C, torch.int32), qe=db("qe", C, torch.int32), te=db("te", C, torch.int32),
-                   qs=db("qs2", C, torch.int32), ts=db("ts2", C, torch.int32), clen=db("cl", C, torch.int32),
-                   counts=db("cn", 4 * C, torch.int32), cstart=db("cs", C, torch.int64),
-                   used=db("used", 1, torch.int64), err=db("err", 1, torch.int32))
+        more = [hb, boff, longest_first(rlen.astype(np.int32), hb)] + ([goff] if goff is not None else [])
+        qd, qo_d, td, to_d, qoff, toff, (hb_p, bo_p, ord_p, *go_p) = self._gather(
+            "s", reads_d, roff, rl, cr, rc, wstart, wlen, more)
+        res = (("score", C, np.int32), ("qe", C, np.int32), ("te", C, np.int32), ("qs", C, np.int32),
+               ("ts", C, np.int32), ("clen", C, np.int32), ("counts", 4 * C, np.int32), ("cstart", C, np.int64),
+               ("used", 1, np.int64), ("err", 1, np.int32))
+        at, nb = packed_layout([n * np.dtype(dt).itemsize for _, n, dt in res])
+        h_res, d_res = self.buf.packed("sw", nb)
+        o = {k: d_res.data_ptr() + x for (k, _, _), x in zip(res, at)}
         cap = int(qoff[-1] + toff[-1] + C)
         cigar = db("cigar", cap, torch.int32)
         need = int(_native.lib().gmf_banded_sw_workspace_bytes(
             C, rlen.astype(np.int32).ctypes.data_as(ctypes.c_void_p),
             wlen.astype(np.int32).ctypes.data_as(ctypes.c_void_p), hb.ctypes.data_as(ctypes.c_void_p), 1))
         sws = db("sws", need, torch.uint8)
-        go_d = up("go", goff, s) if goff is not None else None
-        pairs_c = _native.GmfPairs(C, qd.data_ptr(), qo_d.data_ptr(), td.data_ptr(), to_d.data_ptr(), hb_d.data_ptr(),
-                                   bo_d.data_ptr(), ord_d.data_ptr(), int(hb.max()),
-                                   go_d.data_ptr() if go_d is not None else None, R if goff is not None else 0)
-        sres = _native.GmfSwResults(out["score"].data_ptr(), out["qe"].data_ptr(), out["te"].data_ptr(),
-                                    out["qs"].data_ptr(), out["ts"].data_ptr(), out["counts"].data_ptr(),
-                                    cigar.data_ptr(), cap, out["cstart"].data_ptr(), out["clen"].data_ptr(),
-                                    out["used"].data_ptr(), out["err"].data_ptr())
+        pairs_c = _native.GmfPairs(C, qd.data_ptr(), qo_d.data_ptr(), td.data_ptr(), to_d.data_ptr(), hb_p,
+                                   bo_p, ord_p, int(hb.max()), go_p[0] if go_p else None, R if go_p else 0)
+        sres = _native.GmfSwResults(o["score"], o["qe"], o["te"], o["qs"], o["ts"], o["counts"],
+                                    cigar.data_ptr(), cap, o["cstart"], o["clen"], o["used"], o["err"])
         self._call("gmf_banded_sw", ctypes.byref(pairs_c), ctypes.byref(self.sw), ctypes.byref(sres),
                    ctypes.c_void_p(sws.data_ptr()), need, ctypes.c_void_p(sp))
-        hh = {k: dl("h2_" + k, out[k], n, s) for k, n in
-              (("score", C), ("qe", C), ("te", C), ("qs", C), ("ts", C), ("clen", C), ("counts", 4 * C),
-               ("cstart", C), ("used", 1), ("err", 1))}
+        hh = self._download(h_res, d_res, nb, res, at)
+        early = 4 * cap <= CIGAR_WITH_RESULTS
+        if early:
+            words = self.buf.download("h2_cigar", cigar, cap, s)
         s.synchronize()
         used = int(hh["used"][0])
-        words = dl("h2_cigar", cigar, used, s)
-        s.synchronize()
+        if not early:
+            words = self.buf.download("h2_cigar", cigar, used, s)
+            s.synchronize()
         err = int(hh["err"][0])
         if err:
             raise RuntimeError(f"gmf_banded_sw reported error flags {err}")
         # ExtensionEngine._finish as arrays: reference coordinates from the window start, soft clips from
         # the unaligned ends of the read (copies: the staging buffers are reused by the next batch)
-        qs, qe = hh["qs"][:C].numpy().copy(), hh["qe"][:C].numpy().copy()
-        cols = dict(score=hh["score"][:C].numpy().copy(), qs=qs, qe=qe,
-                    ts=hh["ts"][:C].numpy().astype(np.int64) + wstart,
-                    te=hh["te"][:C].numpy().astype(np.int64) + wstart,
-                    counts=hh["counts"][: 4 * C].numpy().reshape(C, 4).copy(),
-                    cstart=hh["cstart"][:C].numpy().copy(), clen=hh["clen"][:C].numpy().copy(),
-                    clip_l=qs, clip_r=rlen - qe)
+        qs, qe = hh["qs"].copy(), hh["qe"].copy()
+        cols = dict(score=hh["score"].copy(), qs=qs, qe=qe, ts=hh["ts"].astype(np.int64) + wstart,
+                    te=hh["te"].astype(np.int64) + wstart, counts=hh["counts"].reshape(C, 4).copy(),
+                    cstart=hh["cstart"].copy(), clen=hh["clen"].copy(), clip_l=qs, clip_r=rlen - qe)
         if not shared:  # the WFA fallback wants ExtensionResults of these chains
             b = BatchAlignments(C, np.arange(C + 1, dtype=np.int64), cols, words[:used].numpy().view(np.uint32).copy())
             return [b[c][0] for c in range(C)]
@@ -334,7 +358,7 @@ class BatchAligner:
         net = (sp4[:, 3] - sp4[:, 2]) - (sp4[:, 1] - sp4[:, 0])
         wend = np.minimum(self.ref_len, wstart + np.maximum(1, rlen + net))
         wlen = np.maximum(wend - wstart, 0)
-        qd, qo_d, td, to_d, _, _ = self._gather("w", reads_d, roff, rl, cr, rc, wstart, wlen)
+        qd, qo_d, td, to_d, *_ = self._gather("w", reads_d, roff, rl, cr, rc, wstart, wlen)
         dp = DeviceWfaPairs(len(cr), qd, qo_d, td, to_d, rlen.astype(np.int32), wlen.astype(np.int32), self.device)
         res = align_device_pairs(dp, cfg.wfa_max_distance, stream=self.stream,
                                  workspace=lambda nb: self.buf.device_buf("wws", nb, torch.uint8))
