@@ -96,7 +96,8 @@ __global__ void sw_classify_kernel(SwArgs a) {
             p = a.order ? a.order[idx] : idx;
             const int ql = (int)(a.q_off[p + 1] - a.q_off[p]);
             const int tl = (int)(a.t_off[p + 1] - a.t_off[p]);
-            cls = sw_class(ql, tl, a.hb[p], a.m16, a.x16, a.o16, a.e16, a.l8w, a.l16w, a.cmin);
+            // a band beyond the stated widest one is an error that a launched class has to report
+            cls = sw_class(ql, tl, min(a.hb[p], a.max_hb), a.m16, a.x16, a.o16, a.e16, a.l8w, a.l16w, a.cmin);
             a.tb_tag[p] = -1;
             if (a.rm_base) a.rm_base[p] = ~0ull;
         }
