@@ -402,7 +402,7 @@ __device__ __forceinline__ void sw16_rows(const SwArgs& a, const PairGeo& G, boo
     };
 
     // ---- band masks by chunk of the row (32 lanes: chunks 0..32, then the last 33) ----
-    const int n_tab = L == 32 ? imin(nch, MASK_ROWS) : nch;
+    const int n_tab = L == 32 ? imin(nch, a.tabn) : nch;
     for (int x = k; x < n_tab; x += L) {
         const int cc = x <= 32 || L < 32 ? x : x + nch - n_tab;
         unsigned mm[4];
@@ -437,7 +437,10 @@ __device__ __forceinline__ void sw16_rows(const SwArgs& a, const PairGeo& G, boo
     const unsigned codes_at = (unsigned)__cvta_generic_to_shared(sm.codes + (k & 1) * a.tring);
     const unsigned tab_at = (unsigned)__cvta_generic_to_shared(sm.tab);
     int pos = P - VS - 2 * k - 2 * (k & 1);  // ring byte of the chunk's codes
-    int tbi = COOP ? (w - (NW - 1)) * nch * L + k : k;          // word of the chunk's traceback bits
+    // word of the chunk's traceback bits; a cooperative lane moves on to its next strip's words at the row start
+    const int nch_tb = COOP ? sw16_period(W, L) >> 2 : nch;  // chunks of a strip in the words (a padded period has more)
+    const int tb_jump = (NW * nch_tb - nch) * L;
+    int tbi = COOP ? w * nch_tb * L - tb_jump + k : k;
     unsigned tb_lim = COOP ? 0u : (unsigned)(last_chunk + 1) * L;  // no words before a lane's first row
     const unsigned tb_all = (unsigned)(last_chunk + 1) * L;
     const int src = (k + L - 1) & (L - 1);
@@ -575,8 +578,8 @@ __device__ __forceinline__ void sw16_rows(const SwArgs& a, const PairGeo& G, boo
             c.qp = nqp;
             pos += jump;
             if (COOP) {
-                tbi += (NW - 1) * nch * L;
-                tb_lim = tb_all;
+                tbi += tb_jump;
+                tb_lim = min(tb_all, (unsigned)(tbi + nch_tb * L));
             }
             if (XD) {
                 mb = nmb;
@@ -615,7 +618,7 @@ __device__ __forceinline__ void sw16_rows(const SwArgs& a, const PairGeo& G, boo
         for (int gc = 0; gc < n_chunks; ++gc) chunk(gc, True{}, std::integral_constant<int, 16>{});
     } else {
         // rows start in chunks 0..31 of a period and end from chunk nE on and, in the next period, up to chunk 31
-        const int y_jump = 16 * (nch > n_tab ? 34 - (nch - nE) : nE - 32);
+        const int y_jump = 16 * (n_tab - 32 - (nch - nE));
         int gc = 0;
         for (int base = 0;; base += nch) {
             const int e1 = imin(base + 32, n_chunks);
@@ -774,17 +777,20 @@ __global__ void __launch_bounds__(128, L == 16 ? 5 : 4) sw16_kernel(SwArgs a) {
 // lane's output at warp-local step e; warp w reads entry t + 4L of warp w-1
 // at its local step t (t + 4L - P from warp NW-1 for warp 0), so each warp
 // runs at least 4L + 4 steps behind its predecessor, and the cycle of NW
-// warps keeps moving only when P >= NW * (4L + 4) -- the classifier sends a
-// pair here only then.  Under that bound no writer is ever more than P
-// entries ahead of its reader, so the 2- and 4-warp classes use rings of
-// R >= P + 8 entries and no back-pressure.  The 8-warp class (periods up to
-// COOP_PMAX) adds back-pressure instead and keeps 1,024-entry rings: its
-// writers also wait for their readers (see sw16_rows).  Each writer
+// warps keeps moving only when P >= NW * (4L + 4).  A pair with a shorter
+// period than NW * a.coop_lag (4L + 4 and a little slack, so that a warp does
+// not poll at every chunk) is run with this one, its lanes idle between their
+// rows (at most 64 steps, or 16 chunks: the mask table covers a row's last 33).
+// Under that bound no writer is ever more than P entries ahead of its reader,
+// so the 2- and 4-warp classes use rings of R >= P + 8 entries and no
+// back-pressure.  The 8-warp class (periods up to COOP_PMAX) adds
+// back-pressure instead and keeps 1,024-entry rings: its writers also wait
+// for their readers (see sw16_rows).  Each writer
 // publishes its progress after every chunk (ring store, then a release store
 // of the flag); each reader polls the flag with acquire loads and an
 // iteration limit, after which it records GMF_SWF_TIMEOUT and goes on.
-// Traceback words land at the same (global step, lane) positions as in the
-// one-warp layout, so the walk is unchanged.
+// Traceback words land at the same (strip, row step, lane) positions as in
+// the one-warp layout, so the walk is unchanged.
 // ---------------------------------------------------------------------------
 template <int NW, bool TB, bool XD, int EM>
 __device__ void sw16_coop_pair(const SwArgs& a, int p, unsigned char* smem, int* prog, int* cons, int (*sbest)[3],
@@ -799,11 +805,11 @@ __device__ void sw16_coop_pair(const SwArgs& a, int p, unsigned char* smem, int*
         return;
     }
     const int qlen = G.qlen, W = G.W;
-    G.P = sw16_period(W, L);
+    G.P = imax(sw16_period(W, L), NW * a.coop_lag);
     const int P = G.P;
     const int nstrips = (qlen + V - 1) / V;
-    const int my_last = (nstrips - 1) * P + 2 * ((qlen - 1) % V) + W - 1;  // global step of the last cell
-    const int last_chunk = my_last >> 2;
+    // last chunk of the traceback words
+    const int last_chunk = ((nstrips - 1) * sw16_period(W, L) + 2 * ((qlen - 1) % V) + W - 1) >> 2;
 
     const unsigned long long tbw = TB ? sw16_tb_words_l(qlen, W, L) : 0ull;
     if (w == 0) {

@@ -65,9 +65,10 @@ __host__ __device__ inline bool fits_int16(int qlen, int tlen, int m16, int x16,
 // when their period lets that many warps run concurrently (P >= NW * (4*32 +
 // 4)) and the pair has at least two strips per warp.  Each cooperative class
 // covers one period range [NW * 132, 2 * NW * 132) (the 8-warp class up to
-// COOP_PMAX); shorter pairs in those ranges take one warp.
+// COOP_PMAX); shorter pairs in those ranges take one warp.  Periods from
+// `pad_pmin` up to the 2-warp range take two warps as well (see PAD_PMIN).
 __host__ __device__ inline int sw_class(int qlen, int tlen, int hb, int match, int mism, int go, int ge,
-                                        int l8w, int l16w, const int* cmin) {
+                                        int l8w, int l16w, const int* cmin, int pad_pmin) {
     if (!fits_int16(qlen, tlen, match, mism, go, ge)) return CLS_I32;  // scaled scoring (SwArgs m16...)
     const int W = 2 * hb + 1;
     if (W <= l8w) return CLS_I16_L8;
@@ -78,6 +79,7 @@ __host__ __device__ inline int sw_class(int qlen, int tlen, int hb, int match, i
     if (P >= 8 * 132 && P <= COOP_PMAX) return (cmin[2] > 0 && strips >= cmin[2]) ? CLS_I16_C8 : CLS_I16_L32;
     if (P >= 4 * 132 && P < 8 * 132) return (cmin[1] > 0 && strips >= cmin[1]) ? CLS_I16_C4 : CLS_I16_L32;
     if (P >= 2 * 132 && P < 4 * 132) return (cmin[0] > 0 && strips >= cmin[0]) ? CLS_I16_C2 : CLS_I16_L32;
+    if (P >= pad_pmin && P < 2 * 132 && cmin[0] > 0 && strips >= cmin[0]) return CLS_I16_C2;
     return CLS_I16_L32;
 }
 
@@ -97,7 +99,7 @@ __global__ void sw_classify_kernel(SwArgs a) {
             const int ql = (int)(a.q_off[p + 1] - a.q_off[p]);
             const int tl = (int)(a.t_off[p + 1] - a.t_off[p]);
             // a band beyond the stated widest one is an error that a launched class has to report
-            cls = sw_class(ql, tl, min(a.hb[p], a.max_hb), a.m16, a.x16, a.o16, a.e16, a.l8w, a.l16w, a.cmin);
+            cls = sw_class(ql, tl, min(a.hb[p], a.max_hb), a.m16, a.x16, a.o16, a.e16, a.l8w, a.l16w, a.cmin, a.pad_pmin);
             a.tb_tag[p] = -1;
             if (a.rm_base) a.rm_base[p] = ~0ull;
         }
@@ -114,6 +116,25 @@ __global__ void sw_classify_kernel(SwArgs a) {
         }
     }
 }
+
+// Steps by which a warp of a cooperative class lags behind its predecessor at
+// least: 132 let the pipeline move, 8 more let a warp poll every other chunk
+// instead of every one.  One 10 kb pair with periods of 264 / 528 / 1056:
+// 2,344 / 2,147 / 2,827 us at 132, 2,107 / 2,114 / 2,642 at 140, 2,126 / 2,148
+// / 2,701 at 148; 1,184 pairs of 5 kb are within 2% of one another.
+constexpr int COOP_LAG = 140;
+
+// Shortest period that the 2-warp class takes below its own range, run as 2 *
+// COOP_LAG: a pair then takes 140 of the slower cooperative steps a strip
+// instead of a period of one warp's.  That shortens the longest pair's
+// time, and costs a warp that another pair could have had, so it is for
+// batches that leave half the warps idle.  n pairs of 5 kb, W = 209 / 217 /
+// 229 / 241, one warp -> two, us: n = 148: 1,296 / 1,335 / 1,374 / 1,420 ->
+// 1,191 .. 1,196; 592: 1,697 / 1,744 / 1,807 / 1,876 -> 1,845 .. 1,802; 1,184:
+// 2,229 / 2,286 / 2,374 / 2,471 -> 2,267 .. 2,237; serving batches of 1,024
+// mixed reads up to 7% less as a whole (7,349 -> 6,583).
+constexpr int PAD_PMIN = 220;
+static bool few_pairs(int n_pairs, int sms) { return 2ll * n_pairs <= 16ll * sms; }
 
 static size_t round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }
 
@@ -482,6 +503,8 @@ extern "C" int gmf_banded_sw(const gmf_pairs* pairs, const gmf_sw_params* params
     a.l8w = std::min(tun.l8_max_w, L8_WMAX);
     a.l16w = std::min(tun.l16_max_w, L16_WMAX);
     for (int i = 0; i < 3; ++i) a.cmin[i] = tun.coop_min_strips[i];
+    a.pad_pmin = few_pairs(pairs->n_pairs, di.sms) ? PAD_PMIN : 2 * 132;
+    a.coop_lag = COOP_LAG;
 
     const int cls_blocks = std::min((pairs->n_pairs + 255) / 256, di.sms * 4);
     sw_classify_kernel<<<cls_blocks, 256, 0, stream>>>(a);
@@ -521,12 +544,14 @@ extern "C" int gmf_banded_sw(const gmf_pairs* pairs, const gmf_sw_params* params
     const int coop_pcap[3] = {COOP_PMAX, 8 * 132 - 4, 4 * 132 - 4};
     const int coop_knob[3] = {2, 1, 0};  // coop_min_strips index of C8, C4, C2
     for (int c = 0; c < 3; ++c) {
-        if (Pmax < coop_pmin[c] || tun.coop_min_strips[coop_knob[c]] <= 0) continue;  // class empty
+        const bool pad = coop_cls[c] == CLS_I16_C2 && Pmax >= a.pad_pmin;
+        if ((Pmax < coop_pmin[c] && !pad) || tun.coop_min_strips[coop_knob[c]] <= 0) continue;  // class empty
         SwArgs ac = a;
+        const int pcls = std::max(std::min(Pmax, coop_pcap[c]), sw16_coop_warps(coop_cls[c]) * a.coop_lag);
         // the 8-warp class bounds each warp's lead over its reader (1024 entries
         // cover periods up to COOP_PMAX); the others hold a whole period
-        ac.ring = coop_cls[c] == CLS_I16_C8 ? 1024 : ring_entries(std::min(Pmax, coop_pcap[c]) + 7);
-        ac.tring = ring_entries(std::min(Pmax, coop_pcap[c]) + 7);
+        ac.ring = coop_cls[c] == CLS_I16_C8 ? 1024 : ring_entries(pcls + 7);
+        ac.tring = ring_entries(pcls + 7);
         ac.tabn = MASK_ROWS;
         if ((size_t)sw16_coop_warps(coop_cls[c]) * sw16_smem_per_warp(CLS_I16_L32, ac.ring, ac.tring, ac.tabn) + 1024 >
             (size_t)di.smem_optin)

@@ -80,6 +80,8 @@ struct SwArgs {
     unsigned long long* cigar_used;
     int32_t* err;
     int32_t defer_walk;              // batched form: DP kernels leave the walk to sw_walk_kernel
+    int32_t pad_pmin;                // classifier: shortest period that two warps run padded
+    int32_t coop_lag;                // steps that a cooperating warp lags behind its predecessor at least
     int32_t l8w, l16w;               // classifier: widest bands of the 8- and 16-lane classes
     int32_t cmin[3];                 // classifier: fewest strips of the 2-, 4-, 8-warp classes (0: off)
     unsigned long long* tb_base;     // per pair: first traceback word (pool offset)
