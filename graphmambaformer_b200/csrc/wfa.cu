@@ -21,7 +21,7 @@
 //                   long (a side of 4000 codes, or distance 96 when it is
 //                   known): the team's threads take the diagonals of a
 //                   wavefront in turn and extend each one 4, then 8 codes per
-//                   step.
+//                   step, long runs 128 codes per step of their warp.
 //                   The two live wavefronts sit in shared memory (scores up
 //                   to 254 for a warp, 2,049 or 8,205 for a block) and move
 //                   to a global slot beyond.  With a history, wavefront s is also
@@ -33,9 +33,11 @@
 // block has 1,024 threads (a wavefront of 2s+1 diagonals in few turns), a turn
 // compares 4 or 8 codes at once with 32-bit word indices, and the history is
 // kept while the distance is found (in chunks of 32 wavefronts, allocated as
-// the pair goes) instead of replaying every pair to its known distance.  Measured on one B200, 4,000 mixed pairs of 150-20,000 bases:
-// forward 3,711 + 4,061 us (distance, then replay with history) -> 1,654 us,
-// walk 1,091 -> 281 us.
+// the pair goes) instead of replaying every pair to its known distance.  A run
+// of more than 20 matches is finished by the diagonal's whole warp.  Measured
+// on one B200, 4,000 mixed pairs of 150-20,000 bases: forward 3,711 + 4,061 us
+// (distance, then replay with history) -> 1,654 us, with the warps' runs 1,340
+// us; walk 1,091 -> 281 us.
 
 #include <algorithm>
 
@@ -143,10 +145,12 @@ struct Pair {
     }
 };
 
-// Offset after the run of matches from query position i on diagonal k: 4
-// codes (most diagonals stop there), then 8 per step, from aligned words of
-// both sequences.
-__device__ __forceinline__ int wfa_extend(const Pair& P, int i, int k) {
+// Offset after the run of matches from query position i on diagonal k, from
+// aligned words of both sequences: 4 codes (most diagonals stop there), then
+// 8 at a time up to WFA_SHORT codes; `more` when the run goes on (limits of 4,
+// 12, 20 and 28 codes: 2,299 / 2,224 / 2,209 / 2,245 us for the 4,000 pairs).
+constexpr int WFA_SHORT = 20;
+__device__ __forceinline__ int wfa_extend(const Pair& P, int i, int k, bool& more) {
     const int j = i - k;  // (j >= 0 for every offset i >= 0 of a wavefront)
     const int lim = min(P.n - i, P.m - j);
     if (lim <= 0) return i;
@@ -156,7 +160,7 @@ __device__ __forceinline__ int wfa_extend(const Pair& P, int i, int k) {
     unsigned x = P.differing(__funnelshift_r(q0, q1, sq), __funnelshift_r(t0, t1, st));
     if (x) return i + min((__ffs((int)x) - 1) >> 3, lim);
     int adv = 4;
-    while (adv < lim) {
+    while (adv < lim && adv < WFA_SHORT) {
         ++wq;
         ++wt;
         q0 = q1;
@@ -166,14 +170,37 @@ __device__ __forceinline__ int wfa_extend(const Pair& P, int i, int k) {
         t1 = P.T.ld(wt + 1);
         x = P.differing(__funnelshift_r(q0, q1, sq), __funnelshift_r(t0, t1, st));
         const unsigned y = P.differing(__funnelshift_r(q1, q2, sq), __funnelshift_r(t1, t2, st));
-        adv += x ? (__ffs((int)x) - 1) >> 3 : (y ? 4 + ((__ffs((int)y) - 1) >> 3) : 8);
-        if (x | y) break;
+        if (x | y) return i + min(adv + (x ? (__ffs((int)x) - 1) >> 3 : 4 + ((__ffs((int)y) - 1) >> 3)), lim);
+        adv += 8;
         ++wq;
         ++wt;
         q1 = q2;
         t1 = t2;
     }
+    more = adv < lim;
     return i + min(adv, lim);
+}
+
+// The same by the whole warp, 128 codes at a time (i and k are the same in
+// every lane).  Long runs are the few diagonals around the path: one lane
+// would hold up its wavefront for as many steps as the longest of them takes
+// (148 HiFi-like pairs of 15-20 kb: 528 us a call one lane at a time, 245 us
+// so; the 4,000 mixed pairs 2,571 -> 2,209 us).
+__device__ __forceinline__ int wfa_extend_warp(const Pair& P, int i, int k) {
+    const int j = i - k, lim = min(P.n - i, P.m - j), lane = threadIdx.x & 31;
+    int wq = ((P.Q.shift + i) >> 2) + lane, wt = ((P.T.shift + j) >> 2) + lane;
+    const int sq = ((P.Q.shift + i) & 3) * 8, st = ((P.T.shift + j) & 3) * 8;
+    for (int at = 0; at < lim; at += 128, wq += 32, wt += 32) {
+        const unsigned q = __funnelshift_r(P.Q.ld(wq), P.Q.ld(wq + 1), sq);
+        const unsigned t = __funnelshift_r(P.T.ld(wt), P.T.ld(wt + 1), st);
+        const unsigned x = P.differing(q, t);
+        const unsigned b = __ballot_sync(gmf::FULL_MASK, x != 0u);
+        if (b) {
+            const int l = __ffs((int)b) - 1;
+            return i + min(at + 4 * l + ((__ffs((int)__shfl_sync(gmf::FULL_MASK, x, l)) - 1) >> 3), lim);
+        }
+    }
+    return i + max(lim, 0);
 }
 
 // A pair is computed by one warp, or by the whole block when it is long.
@@ -219,7 +246,7 @@ __device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm
         P.plain = !tm.sync_any(other);
     }
     long long h0 = 0;
-    if (tm.rank == 0) h0 = wfa_extend(P, 0, 0);
+    if (tm.rank < 32) h0 = wfa_extend_warp(P, 0, 0);
     h0 = tm.bcast0(h0, scratch);
     long long chunk = -1;
     int* row = nullptr;  // wavefront s is kept at row[k]
@@ -263,18 +290,30 @@ __device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm
         const int hi = MODE == KNOWN ? min(s, final_k + (limit - s)) : s;
         bool done = false;
         if (tm.rank < 4) cur[cen + (tm.rank < 2 ? -s - 2 + tm.rank : s - 1 + tm.rank)] = WFA_NONE;
-        for (int k = lo + tm.rank; k <= hi; k += Team::SIZE) {
+        const int lane = threadIdx.x & 31;
+        for (int kw = lo + tm.rank - lane; kw <= hi; kw += Team::SIZE) {  // a warp's 32 diagonals
+            const int k = kw + lane;
+            const bool mine = k <= hi;
             // a candidate past the end of a sequence is none (before the start it cannot be)
             const int top = min(n, m + k);
-            int sub = prev[k + cen] + 1, ins = prev[k - 1 + cen] + 1, del = prev[k + 1 + cen];
+            int sub = WFA_NONE, ins = WFA_NONE, del = WFA_NONE;
+            if (mine) sub = prev[k + cen] + 1, ins = prev[k - 1 + cen] + 1, del = prev[k + 1 + cen];
             sub = sub <= top ? sub : WFA_NONE;
             ins = ins <= top ? ins : WFA_NONE;
             del = del <= top ? del : WFA_NONE;
             const int best = max(max(sub, ins), del);
-            const int r = best >= 0 ? wfa_extend(P, best, k) : WFA_NONE;
-            cur[k + cen] = r;
-            if (MODE != DIST && (MODE == KNOWN || row)) row[k] = r;
-            done |= (k == final_k) && r >= n;
+            bool more = false;
+            int r = best >= 0 ? wfa_extend(P, best, k, more) : WFA_NONE;
+            for (unsigned b = __ballot_sync(gmf::FULL_MASK, more); b; b &= b - 1) {
+                const int l = __ffs((int)b) - 1;
+                const int e = wfa_extend_warp(P, __shfl_sync(gmf::FULL_MASK, r, l), kw + l);
+                if (lane == l) r = e;
+            }
+            if (mine) {
+                cur[k + cen] = r;
+                if (MODE != DIST && (MODE == KNOWN || row)) row[k] = r;
+                done |= (k == final_k) && r >= n;
+            }
         }
         return tm.sync_any(done);
     };
