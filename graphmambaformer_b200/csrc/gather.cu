@@ -24,10 +24,23 @@ __global__ void __launch_bounds__(256) gather_segments_kernel(const int8_t* __re
         const int L = len[i];
         const bool rev = rc != nullptr && rc[i] != 0;
         int8_t* d = dst + dst_off[i];
-        for (int x = threadIdx.x; x < L; x += blockDim.x) {
-            const int64_t pos = rev ? s + (L - 1 - x) : s + x;
-            const int8_t c = (pos >= 0 && pos < src_len) ? src[pos] : (int8_t)-1;
-            d[x] = rev ? complement_code(c) : c;
+        // The time is that of the longest segment's loads, one after another
+        // in its block, so 8 are in flight per thread (1,024 reads of 150 bp
+        // to 20 kb: 44 -> 14 us, their windows 29 -> 13 us).
+        constexpr int U = 8;
+        for (int x0 = threadIdx.x; x0 < L; x0 += U * (int)blockDim.x) {
+            int8_t c[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int x = x0 + u * (int)blockDim.x;
+                const int64_t pos = rev ? s + (L - 1 - x) : s + x;
+                c[u] = (x < L && pos >= 0 && pos < src_len) ? src[pos] : (int8_t)-1;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int x = x0 + u * (int)blockDim.x;
+                if (x < L) d[x] = rev ? complement_code(c[u]) : c[u];
+            }
         }
     }
 }
