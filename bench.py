@@ -244,15 +244,26 @@ def load_traffic():
     return out
 
 
-def launches_per_call(max_half_band: int, traceback: bool) -> int:
-    """Kernels one gmf_banded_sw call launches: the classifier, one kernel per
-    pair class that can be populated (the cooperative classes only when the
-    widest band reaches their period range), and the deferred walk."""
+def launches_per_call(max_half_band: int, traceback: bool, n_pairs: int) -> int:
+    """Kernels one gmf_banded_sw call launches under the current tuning: the
+    classifier, one kernel per pair class that the widest band leaves
+    possible (two warps also below their period range in a batch that leaves
+    half the warps idle), the int32 class and the deferred walk."""
+    import ctypes
+
+    import torch
+
+    from graphmambaformer_b200 import _native
+
+    t = _native.GmfSwTuning()
+    _native.check("gmf_sw_get_tuning", _native.lib().gmf_sw_get_tuning(ctypes.byref(t)))
     W = 2 * max_half_band + 1
-    P = max(W + 2, 128)
-    P = (P + 3) & ~3
-    coop = sum(1 for pmin in (8 * 132, 4 * 132, 2 * 132) if P >= pmin)
-    return 1 + coop + 3 + 1 + (1 if traceback else 0)
+    P = (max(W + 2, 128) + 3) & ~3
+    few = 2 * n_pairs <= 16 * torch.cuda.get_device_properties(0).multi_processor_count
+    pmin = (220 if few else 2 * 132, 4 * 132, 8 * 132)
+    coop = sum(1 for i in range(3) if P >= pmin[i] and t.coop_min_strips[i] > 0)
+    l8, l16 = min(t.l8_max_w, 1021), min(t.l16_max_w, 2045)
+    return 1 + coop + 1 + (W > l8) + (W > l16) + 1 + (1 if traceback else 0)
 
 
 def time_device(fn, steps, stream, flush):
@@ -444,7 +455,7 @@ def run_b200(args):
         pp = max_over_ranks(pipe) if pipe is not None else None
         return dict(ps=ps, params=params, desc=desc, cells=cells, total=total, batched_ms=b, graph_ms=gr, plain_ms=pl,
                     e2e_ms=c2, sync_ms=c, session_ms=e, pipelined_ms=pp, rank_ms=float(np.mean(b_ms)),
-                    sess_io=sess_io, ctx_io=ctx_io, launches=launches_per_call(dp.max_half_band, True),
+                    sess_io=sess_io, ctx_io=ctx_io, launches=launches_per_call(dp.max_half_band, True, len(ps)),
                     result=result)
 
     # ---- autotuned scheduling of the batched form (on a 10% sample of the
@@ -517,7 +528,7 @@ def run_b200(args):
         chain = {
             "value": anchors_total / (c_ms * 1e-3), "unit": "anchors/s", "ms_per_step": c_ms,
             "pair_evaluations_per_step": evals,
-            "config": cdesc, "gpu_launches_per_step": 3,
+            "config": cdesc, "gpu_launches_per_step": 6,  # two sorts, DP, two one-chain passes, peel
             "e2e": {"value": anchors_total / (ce_ms * 1e-3), "unit": "anchors/s", "ms_per_step": ce_ms,
                     "h2d_bytes_per_step": csess.h2d_bytes, "d2h_bytes_per_step": csess.d2h_bytes},
         }

@@ -515,9 +515,8 @@ extern "C" int gmf_banded_sw(const gmf_pairs* pairs, const gmf_sw_params* params
     // The first class kernel goes to the caller's stream, every other one to a
     // side stream of its own (or, untuned-off, to the caller's stream too),
     // longest classes first; classes that the widest band rules out are not
-    // launched.  Pairs of 150 bp, with every class on a side stream, several
-    // of them empty, and four memsets before them: 124 us for 2,000 and 180 us
-    // for 10,000; so: 76 and 170 us.
+    // launched.  10,000 pairs of 150 bp: 180 us with every class on a side
+    // stream, several of them empty, and four memsets before them; so: 170 us.
     SideStreams* ss = nullptr;
     const bool fork = tun.side_streams != 0;
     if (fork) {
