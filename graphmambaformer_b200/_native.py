@@ -262,6 +262,7 @@ _SIGNATURES = {
     "gmf_sw_get_tuning": (c_int, [POINTER(GmfSwTuning)]),
     "gmf_sw_set_tuning": (c_int, [POINTER(GmfSwTuning)]),
     "gmf_sw_test_coop_wait": (c_int, [c_int32, c_int32]),
+    "gmf_sw_test_delay_ring": (c_int, [c_int32, c_int32, POINTER(c_int32), POINTER(c_int32)]),
     "gmf_chain_dp": (c_int, [c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32,
                              c_int32, c_void_p, c_int32, c_void_p, c_void_p, c_void_p]),
     "gmf_chain_sort": (c_int, [POINTER(GmfAnchorBatch), POINTER(GmfSortedAnchors), c_void_p,

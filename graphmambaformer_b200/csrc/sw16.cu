@@ -32,10 +32,12 @@
 //
 // Steps run in chunks of 4, and rows always start on a chunk boundary, so
 // once per chunk a lane: reads one word of target codes from a shared ring,
-// reads 4 delay-line entries with one 16-byte shared-memory access, stores
-// one 32-bit traceback word (4 bits per cell), and checks the chunk's maxima
-// for the best cell (the first maximum in row-then-slot order is recovered
-// from the chunk's 4 kept H values when the maximum grows).
+// reads 4 delay-line entries with one 16-byte shared-memory access (from a
+// ring one chunk longer than the line, so that it never shares a slot with the
+// chunk's own stores), stores one 32-bit traceback word (4 bits per cell), and
+// checks the chunk's maxima for the best cell (the first maximum in
+// row-then-slot order is recovered from the chunk's 4 kept H values when the
+// maximum grows).
 //
 // Long pairs with wide bands run in the cooperative form below: the warps of
 // one CTA share a pair strip by strip.

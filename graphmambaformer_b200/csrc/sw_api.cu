@@ -221,6 +221,12 @@ static int ring_entries(int d_max) {
     return r;
 }
 
+// Entries of the 16x2 form's delay line (D = P - 4L steps; one more chunk than
+// it holds): a chunk's last lane stores entries 4g .. 4g+3 while its first lane
+// reads 4g-D .. 4g-D+3, and nothing orders the two within the chunk, so they
+// never share a slot; the chunks themselves are a warp barrier apart.
+static int delay_ring(int period, int lanes) { return ring_entries(period - 4 * lanes + 3); }
+
 static int check_common(const gmf_pairs* pairs, const gmf_sw_params* params, const gmf_sw_results* res) {
     if (!pairs || !params || !res) return GMF_ERR_INVALID_ARGUMENT;
     if (pairs->n_pairs < 0) return GMF_ERR_INVALID_ARGUMENT;
@@ -567,7 +573,7 @@ extern "C" int gmf_banded_sw(const gmf_pairs* pairs, const gmf_sw_params* params
         const int L = lanes[c];
         if (c > 0 && Wmax <= (c == 2 ? a.l16w : a.l8w)) continue;  // class empty
         SwArgs ac = a;
-        ac.ring = ring_entries(std::max(3, sw16_period(cls_wmax[c], L) - 4 * L - 1));
+        ac.ring = delay_ring(sw16_period(cls_wmax[c], L), L);
         ac.tring = ring_entries(sw16_period(cls_wmax[c], L) + 7);
         ac.tabn = L == 32 ? MASK_ROWS : sw16_period(cls_wmax[c], L) / 4;
         const int wpb = warps_per_block((size_t)sw16_smem_per_warp(c, ac.ring, ac.tring, ac.tabn), di,
@@ -646,5 +652,14 @@ extern "C" int gmf_sw_test_coop_wait(int32_t spin_limit, int32_t stall_writers) 
     if (spin_limit < 0 || (stall_writers != 0 && stall_writers != 1)) return GMF_ERR_INVALID_ARGUMENT;
     g_test_spin_limit.store(spin_limit);
     g_test_stall.store(stall_writers);
+    return GMF_OK;
+}
+
+extern "C" int gmf_sw_test_delay_ring(int32_t half_band, int32_t lanes, int32_t* delay, int32_t* entries) {
+    if (half_band < 0 || half_band > GMF_MAX_HALF_BAND || (lanes != 8 && lanes != 16 && lanes != 32) || !delay || !entries)
+        return GMF_ERR_INVALID_ARGUMENT;
+    const int P = sw16_period(2 * half_band + 1, lanes);
+    *delay = P - 4 * lanes;
+    *entries = delay_ring(P, lanes);
     return GMF_OK;
 }

@@ -281,6 +281,12 @@ int gmf_sw_set_tuning(const gmf_sw_tuning* tuning);
  * gmf_banded_sw call in the process until reset with (0, 0). */
 int gmf_sw_test_coop_wait(int32_t spin_limit, int32_t stall_writers);
 
+/* Test hook of the delay line of the one-warp classes (no counterpart in the
+ * reference): the steps a lane group of `lanes` (8, 16 or 32) delays its last
+ * row by for pairs of this half band, and the ring entries that
+ * gmf_banded_sw gives the line.  Host only. */
+int gmf_sw_test_delay_ring(int32_t half_band, int32_t lanes, int32_t* delay, int32_t* entries);
+
 /* ======================================================================== */
 /* Anchor chaining                                                          */
 /* ======================================================================== */
