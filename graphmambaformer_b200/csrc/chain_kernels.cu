@@ -876,8 +876,8 @@ struct PeelArgs {
 // children, so a warp per block of 32 nodes collects each node's ancestors
 // inside the block as a bit mask, and the first ancestor before it, in five
 // rounds of doubling; one thread then hops block by block.  A read for which
-// the bounds do not hold (several chains above the cutoff, negative scores,
-// too few members) is left to the general form below, n_chains = PENDING.
+// the bounds do not hold (several chains above the cutoff, negative scores or
+// limits, too few members) is left to the general form below, n_chains = PENDING.
 //
 // What bounds it is reading f, parents and positions once; the general form
 // ranks every possible start and walks them in one thread.  Measured on one
@@ -954,8 +954,8 @@ __device__ void one_chain(const PeelArgs& a, int r, unsigned char* smem) {
     int state = PENDING;
     if (ns[0] == 0 && ns[1] == 0)
         state = 0;
-    else if (!(mn >= 0.0) || !(a.secondary_score_ratio >= 0.0) || n > CAP)
-        state = PENDING;
+    else if (!(mn >= 0.0) || !(a.secondary_score_ratio >= 0.0) || 0.0 > a.secondary_overlap || n > CAP)
+        state = PENDING;  // (an overlap limit below 0 drops the best chain too)
     else if (!(best >= a.min_chain_score))
         state = 0;  // no walk scores more than its start
     else if (ns[1 - g] == 0 || mx[1 - g] < cutoff)
