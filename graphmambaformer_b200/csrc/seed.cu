@@ -229,6 +229,7 @@ struct TileArgs {
     SeedArgs s;
     int bits;               // prefix table (0: none)
     const int32_t* first;
+    long long total;        // codes that may be read
     long long slots;        // tile slots the workspace holds
     int32_t* n_sel;         // per slot: selected k-mers, forward and reverse
     long long* n_anchor;    // per slot: anchors, forward and reverse
@@ -238,10 +239,17 @@ struct TileArgs {
     const long long* off;   // emit: anchor offsets
 };
 
+// A read's first code.  The workspace holds the slots of `total` codes, so a
+// read that goes on beyond them is cut there.
+__device__ __forceinline__ long long tile_off(const TileArgs& a, int r) {
+    const long long o = a.s.read_off[r];
+    return o < a.total ? o : a.total;
+}
+
 // Read r owns the tile slots from (its offset) / TILE + r on: at least as many
 // as it has tiles, and never more than total / TILE + n_reads in all.
 __device__ __forceinline__ long long first_slot(const TileArgs& a, int r) {
-    return (a.s.read_off[r] - a.s.read_off[0]) / TILE + r;
+    return (tile_off(a, r) - tile_off(a, 0)) / TILE + r;
 }
 
 // The read of a slot: the last r with first_slot(r) <= slot.  32 reads are
@@ -333,8 +341,8 @@ __global__ void __launch_bounds__(TILE_THREADS) seed_tile_kernel(TileArgs a) {
         }
         __syncthreads();
         const int r = s_read;
-        const long long r0 = a.s.read_off[r];
-        const int L = (int)(a.s.read_off[r + 1] - r0);
+        const long long r0 = tile_off(a, r);
+        const int L = (int)(tile_off(a, r + 1) - r0);
         const int m = L - k + 1;  // k-mer positions
         const long long t0l = (slot - first_slot(a, r)) * TILE;
         if (t0l >= m) {  // a slot beyond the read's tiles (or past the last read)
@@ -562,7 +570,7 @@ __global__ void __launch_bounds__(128) seed_emit_kernel(TileArgs a) {
         }
         __syncthreads();
         const int r = s_read;
-        const int m = (int)(a.s.read_off[r + 1] - a.s.read_off[r]) - a.s.k + 1;
+        const int m = (int)(tile_off(a, r + 1) - tile_off(a, r)) - a.s.k + 1;
         const long long first = first_slot(a, r), last = first + (m - 1) / TILE;
         // anchors of the read's tiles before this one, in the orientation's order
         long long before = 0;
@@ -644,6 +652,7 @@ size_t carve_tiles(int n_reads, long long total, char* ws, TileArgs& a) {
         at += up256(bytes);
         return p;
     };
+    a.total = total;
     a.slots = (long long)S;
     a.counts = (long long*)take(2 * (size_t)n_reads * 8);
     a.n_anchor = (long long*)take(2 * S * 8);

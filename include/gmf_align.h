@@ -230,8 +230,8 @@ typedef struct {
 
 int gmf_seed_prefix_fill(const gmf_minimizer_index* index, int32_t bits, int32_t* first, gmf_stream_t stream);
 
-/* total_codes: host value >= read_off[n_reads] (codes beyond it are not read
- * and find no anchors). */
+/* total_codes: host value >= read_off[n_reads].  Codes beyond it are not read:
+ * a read that goes on is cut there. */
 size_t gmf_seed_workspace_bytes(int32_t n_reads, int64_t total_codes);
 
 /* Scan: anchor_off[2 * n_reads + 1] receives the anchor offsets (per read
