@@ -123,6 +123,30 @@ __device__ __forceinline__ long long chunk_row(int s) {
     return 2 + (long long)s * s - s0 * s0;
 }
 
+// Chunks of a pair's own share of the history: those of about 8% differences,
+// as the caller sizes the workspace.
+__device__ __forceinline__ int history_share(int longest, int bound) {
+    return min(min(longest, bound), (int)(longest * 8ll / 100) + 48) / WFA_CHUNK + 1;
+}
+
+// The place of a pair's chunk c in the history, or -1 when it does not fit.
+// A pair takes its own share as long as there is room, and more only while
+// half of the room is left, so that a few unrelated pairs do not use up the
+// others' shares (160 of 4.1 kb before 64 related ones of 300 bases, in a
+// workspace of their shares: the 64 found nothing left).  A chunk that does
+// not fit gives its place back, for smaller ones: the one request that crosses
+// the end sets the counter back, every other one until then starts beyond the
+// end and is refused.  (Taken by compare and swap instead, one chunk at a
+// time, the 4,000 first chunks alone cost 3 ms.)
+__device__ __forceinline__ long long take_chunk(const WfaArgs& A, int c, int own) {
+    const long long need = chunk_ints(c);
+    if (c >= own && (long long)*(volatile unsigned long long*)A.hist_used + need > A.hist_cap / 2) return -1;
+    const long long o = (long long)atomicAdd(A.hist_used, (unsigned long long)need);
+    if (o + need <= A.hist_cap) return o;
+    if (o <= A.hist_cap) atomicExch(A.hist_used, (unsigned long long)o);
+    return -1;
+}
+
 // Bytes of a that match nothing (N = 5, negative), as their top bits; those
 // above the lowest may be false.
 __device__ __forceinline__ unsigned unmatched(unsigned a) {
@@ -250,14 +274,12 @@ __device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm
     h0 = tm.bcast0(h0, scratch);
     long long chunk = -1;
     int* row = nullptr;  // wavefront s is kept at row[k]
+    const int own = MODE == CHUNKED ? history_share(max(n, m), limit) : 0;
     auto next_chunk = [&](int s) {  // the chunk that starts with wavefront s
-        long long o = 0;
+        long long o = -1;
         if (tm.rank == 0) {
-            const long long need = chunk_ints(s / WFA_CHUNK);
-            o = (long long)atomicAdd(A.hist_used, (unsigned long long)need);
-            if (o + need > A.hist_cap) {
-                o = -1;
-            } else {
+            o = take_chunk(A, s / WFA_CHUNK, own);
+            if (o >= 0) {
                 A.hist[o] = (int)(unsigned)(unsigned long long)chunk;
                 A.hist[o + 1] = (int)(unsigned)((unsigned long long)chunk >> 32);
             }

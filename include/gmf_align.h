@@ -601,8 +601,11 @@ int gmf_wfa_align(const gmf_wfa_pairs* pairs, const int32_t* distance, int32_t m
 /* Distance and CIGAR of every pair in one pass: the wavefronts are kept while
  * the distance is found, in chunks of 32 (2 + 1024 (2c + 1) ints for
  * wavefronts 32c .. 32c + 31) taken from the workspace's history entries
- * (gmf_wfa_workspace_bytes).  Pairs whose chunks do not fit still get their
- * distance, and cigar_len[p] = -2: gmf_wfa_align gives their CIGARs. */
+ * (gmf_wfa_workspace_bytes).  A pair's own share of them is its chunks up to
+ * distance min(L, max_distance, 8 L / 100 + 48), L its longer side; beyond it
+ * a pair takes chunks only while half of the entries are left, so at least
+ * that half is kept for the shares.  Pairs whose chunks do not fit still get
+ * their distance, and cigar_len[p] = -2: gmf_wfa_align gives their CIGARs. */
 int gmf_wfa_align_direct(const gmf_wfa_pairs* pairs, int32_t max_distance, int32_t* distance,
                          const gmf_wfa_results* results, void* workspace, size_t workspace_bytes,
                          gmf_stream_t stream);
