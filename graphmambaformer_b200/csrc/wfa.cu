@@ -24,7 +24,12 @@
 //                   step, long runs 128 codes per step of their warp.
 //                   The two live wavefronts sit in shared memory (scores up
 //                   to 254 for a warp, 2,049 or 8,205 for a block) and move
-//                   to a global slot beyond.  With a history, wavefront s is also
+//                   to a global slot beyond: one per block where its shared
+//                   memory may not do, and 16-bit ones that the warps claim as
+//                   they need them (a side of theirs is below 4000, so 148
+//                   blocks of 32 warps need 152 MB for any bound, 64 pairs 2 MB;
+//                   a 32-bit slot of the whole bound for every warp of every
+//                   block took 311 and 134 MB at 4,096).  With a history, wavefront s is also
 //                   stored, for the walk.
 //   walk kernel     one warp per pair, from the last wavefront back.
 //
@@ -48,10 +53,11 @@ namespace {
 constexpr int WFA_SMEM_S = 254;                       // a warp's wavefronts up to this score in shared memory
 constexpr int WFA_SMEM_WF = 2 * WFA_SMEM_S + 5;       // ints per shared wavefront (two sentinels at each end)
 constexpr int WFA_NONE = -(1 << 30);                  // no offset: stays negative after the + 1 of a candidate
+constexpr int WFA_NONE16 = -(1 << 14);                // the same in 16 bits
 constexpr int WFA_LONG_LEN = 4000;  // distance unknown: a pair with a side this long gets a whole block
 constexpr int WFA_LONG_D = 96;      // distance known: a pair at this distance gets a whole block
 constexpr int WFA_WIDE = 1024;      // threads of a block when its wavefronts always fit its shared memory
-constexpr int WFA_NARROW = 256;     // and beyond (half the global slots)
+constexpr int WFA_NARROW = 256;     // and beyond
 constexpr int WFA_CHUNK = 32;       // wavefronts per history chunk
 
 __host__ __device__ constexpr int block_scores(int threads) { return (threads / 32 * WFA_SMEM_WF - 5) / 2; }
@@ -97,7 +103,10 @@ struct WfaArgs {
     Seq Q, T;
     int max_distance;
     int eff;               // largest distance any pair can reach: min(max_distance, longest side)
-    int* spill;            // 2 * (2*eff + 5) ints per warp, or null when eff <= WFA_SMEM_S
+    int warp_eff;          // the same for a pair of one warp
+    int* block_spill;      // 2 * (2*eff + 5) ints per block, or null where its shared memory holds every score
+    short* warp_spill;     // slots of 2 * (2*warp_eff + 5), or null when warp_eff <= WFA_SMEM_S
+    unsigned* warp_slots;  // slots claimed
     unsigned* work;        // pair counters of the forward and the walk kernel
     int* distance;         // written, or read when the history is replayed (KNOWN)
     int* hist;
@@ -227,10 +236,20 @@ __device__ __forceinline__ int wfa_extend_warp(const Pair& P, int i, int k) {
     return i + max(lim, 0);
 }
 
-// A pair is computed by one warp, or by the whole block when it is long.
+// A pair is computed by one warp, or by the whole block when it is long.  A
+// team keeps wavefronts beyond its shared memory as Spilled, in spill().
 struct WarpTeam {
     int rank;
+    int* slot;  // shared memory: the warp's slot, -1 until it needs one
     static constexpr int SIZE = 32;
+    using Spilled = short;
+    __device__ int top(const WfaArgs& A) const { return A.warp_eff; }
+    // At most one slot per warp that computes pairs: no more than there are warps, or pairs.
+    __device__ short* spill(const WfaArgs& A) const {
+        if (rank == 0 && *slot < 0) *slot = (int)atomicAdd(A.warp_slots, 1u);
+        __syncwarp();
+        return A.warp_spill + (long long)*slot * (2 * (2 * A.warp_eff + 5));
+    }
     __device__ void sync() const { __syncwarp(); }
     __device__ bool sync_any(bool x) const {
         __syncwarp();
@@ -243,6 +262,11 @@ template <int T>
 struct BlockTeam {
     int rank;
     static constexpr int SIZE = T;
+    using Spilled = int;
+    __device__ int top(const WfaArgs& A) const { return A.eff; }
+    __device__ int* spill(const WfaArgs& A) const {
+        return A.block_spill + (long long)blockIdx.x * (2 * (2 * A.eff + 5));
+    }
     __device__ void sync() const { __syncthreads(); }
     __device__ bool sync_any(bool x) const { return __syncthreads_or(x) != 0; }
     __device__ long long bcast0(long long v, long long* scratch) const {
@@ -254,15 +278,19 @@ struct BlockTeam {
     }
 };
 
+__device__ __forceinline__ void put_offset(int* at, int v) { *at = v; }
+__device__ __forceinline__ void put_offset(short* at, int v) { *at = (short)max(v, WFA_NONE16); }
+
 // The wavefronts of one pair up to completion; returns the distance, or -1
 // once `limit` is reached without completing.  `sm` holds two wavefronts of
-// scores up to `sm_s`; beyond that they move to `gl` (two of 2*eff+3).
+// scores up to `sm_s`; beyond that they move to the team's global slot (two of
+// 2*top+5).
 // KNOWN: `hist` is the pair's history, and only the diagonals that can still
 // reach the end by `limit` (the distance) are computed.  CHUNKED: *last
 // receives the offset of the last chunk, -1 when the workspace ran out.
 template <Mode MODE, class Team>
-__device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm_s, int* gl, int* hist,
-                           long long* last, const Team& tm, long long* scratch) {
+__device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm_s, int* hist, long long* last,
+                           const Team& tm, long long* scratch) {
     const int n = P.n, m = P.m, final_k = n - m;
     {
         bool other = false;  // (bytes around the query's ends only make the pair look less plain)
@@ -299,7 +327,7 @@ __device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm
     if (tm.rank < 5) sm[cen - 2 + tm.rank] = tm.rank == 2 ? (int)h0 : WFA_NONE;
     tm.sync();
     // One wavefront from the one before; true when the pair is complete.
-    auto wave = [&](int s, const int* prev, int* cur) {
+    auto wave = [&](int s, const auto* prev, auto* cur) {
         if (MODE == CHUNKED) {
             if ((s & (WFA_CHUNK - 1)) == 0 && chunk >= 0) {
                 next_chunk(s);
@@ -311,7 +339,7 @@ __device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm
         const int lo = MODE == KNOWN ? max(-s, final_k - (limit - s)) : -s;
         const int hi = MODE == KNOWN ? min(s, final_k + (limit - s)) : s;
         bool done = false;
-        if (tm.rank < 4) cur[cen + (tm.rank < 2 ? -s - 2 + tm.rank : s - 1 + tm.rank)] = WFA_NONE;
+        if (tm.rank < 4) put_offset(cur + cen + (tm.rank < 2 ? -s - 2 + tm.rank : s - 1 + tm.rank), WFA_NONE);
         const int lane = threadIdx.x & 31;
         for (int kw = lo + tm.rank - lane; kw <= hi; kw += Team::SIZE) {  // a warp's 32 diagonals
             const int k = kw + lane;
@@ -332,7 +360,7 @@ __device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm
                 if (lane == l) r = e;
             }
             if (mine) {
-                cur[k + cen] = r;
+                put_offset(cur + k + cen, r);
                 if (MODE != DIST && (MODE == KNOWN || row)) row[k] = r;
                 done |= (k == final_k) && r >= n;
             }
@@ -341,26 +369,28 @@ __device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm
     };
     int s = 1;
     int *prev = sm, *cur = sm + 2 * sm_s + 5;
+    const int top = tm.top(A);  // s <= max(n, m) <= top always holds
     for (; s <= sm_s; ++s) {
-        if (s - 1 >= limit || s > A.eff) return -1;  // s <= max(n, m) <= eff always holds
+        if (s - 1 >= limit || s > top) return -1;
         if (wave(s, prev, cur)) return s;
         int* tmp = prev;
         prev = cur;
         cur = tmp;
     }
-    if (s - 1 >= limit || s > A.eff) return -1;
+    if (s - 1 >= limit || s > top) return -1;
     // the live wavefront moves to the global slot
+    typename Team::Spilled* gprev = tm.spill(A);
+    typename Team::Spilled* gcur = gprev + 2 * top + 5;
     {
-        const int gcen = A.eff + 2, k0 = -(s - 1) - 2;
-        for (int k = k0 + tm.rank; k <= -k0; k += Team::SIZE) gl[k + gcen] = prev[k + cen];
+        const int gcen = top + 2, k0 = -(s - 1) - 2;
+        for (int k = k0 + tm.rank; k <= -k0; k += Team::SIZE) put_offset(gprev + k + gcen, prev[k + cen]);
         cen = gcen;
     }
     tm.sync();
-    int *gprev = gl, *gcur = gl + 2 * A.eff + 5;
     for (;; ++s) {
-        if (s - 1 >= limit || s > A.eff) return -1;
+        if (s - 1 >= limit || s > top) return -1;
         if (wave(s, gprev, gcur)) return s;
-        int* tmp = gprev;
+        auto* tmp = gprev;
         gprev = gcur;
         gcur = tmp;
     }
@@ -369,15 +399,14 @@ __device__ int wfa_forward(const WfaArgs& A, Pair& P, int limit, int* sm, int sm
 // One pair: its distance, its distance and history, or the history of its
 // known distance.
 template <Mode MODE, class Team>
-__device__ void wfa_pair(const WfaArgs& A, int p, int* sm, int sm_s, int* gl, const Team& tm, long long* scratch) {
+__device__ void wfa_pair(const WfaArgs& A, int p, int* sm, int sm_s, const Team& tm, long long* scratch) {
     const long long q0 = A.q_off[p], t0 = A.t_off[p];
     const int n = (int)(A.q_off[p + 1] - q0), m = (int)(A.t_off[p + 1] - t0);
     Pair P(A.Q, q0, n, A.T, t0, m);
     if (MODE != KNOWN) {
         long long last = -1;
         const int d = n == 0 || m == 0 ? max(n, m)
-                                       : wfa_forward<MODE>(A, P, A.max_distance, sm, sm_s, gl, nullptr, &last, tm,
-                                                           scratch);
+                                       : wfa_forward<MODE>(A, P, A.max_distance, sm, sm_s, nullptr, &last, tm, scratch);
         if (tm.rank == 0) {
             A.distance[p] = d;
             if (MODE == CHUNKED) A.hist_off[p] = last;
@@ -399,7 +428,7 @@ __device__ void wfa_pair(const WfaArgs& A, int p, int* sm, int sm_s, int* gl, co
         }
         off = tm.bcast0(off, scratch);
         if (off >= 0) {
-            const int got = wfa_forward<KNOWN>(A, P, d, sm, sm_s, gl, A.hist + off, nullptr, tm, scratch);
+            const int got = wfa_forward<KNOWN>(A, P, d, sm, sm_s, A.hist + off, nullptr, tm, scratch);
             if (got != d) off = -1;  // cannot happen: the pass is deterministic
         }
     }
@@ -422,12 +451,10 @@ template <Mode MODE, int T>
 __global__ void __launch_bounds__(T, T == WFA_WIDE ? 1 : 2) wfa_forward_kernel(WfaArgs A) {
     constexpr int WARPS = T / 32;
     extern __shared__ int s_wf[];
-    __shared__ int s_pos[WARPS];
+    __shared__ int s_pos[WARPS], s_slot[WARPS];
     __shared__ long long s_scratch;
     const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
-    const long long slot = 2 * (2ll * A.eff + 5);
-    int* gl_warp = A.spill ? A.spill + ((long long)blockIdx.x * WARPS + wib) * slot : nullptr;
-    int* gl_block = A.spill ? A.spill + (long long)blockIdx.x * WARPS * slot : nullptr;
+    if (lane == 0) s_slot[wib] = -1;
     const unsigned n = (unsigned)A.n_pairs;
     for (;;) {
         if (tid == 0) {
@@ -450,7 +477,7 @@ __global__ void __launch_bounds__(T, T == WFA_WIDE ? 1 : 2) wfa_forward_kernel(W
             if (s_pos[e] < 0) continue;
             const int p = A.order ? A.order[s_pos[e]] : s_pos[e];
             if (wfa_is_long<MODE>(A, p)) {
-                wfa_pair<MODE>(A, p, s_wf, block_scores(T), gl_block, BlockTeam<T>{tid}, &s_scratch);
+                wfa_pair<MODE>(A, p, s_wf, block_scores(T), BlockTeam<T>{tid}, &s_scratch);
                 any_long = true;
                 __syncthreads();
             }
@@ -459,7 +486,8 @@ __global__ void __launch_bounds__(T, T == WFA_WIDE ? 1 : 2) wfa_forward_kernel(W
         if (s_pos[wib] >= 0) {
             const int p = A.order ? A.order[s_pos[wib]] : s_pos[wib];
             if (!wfa_is_long<MODE>(A, p))
-                wfa_pair<MODE>(A, p, s_wf + wib * 2 * WFA_SMEM_WF, WFA_SMEM_S, gl_warp, WarpTeam{lane}, nullptr);
+                wfa_pair<MODE>(A, p, s_wf + wib * 2 * WFA_SMEM_WF, WFA_SMEM_S, WarpTeam{lane, s_slot + wib},
+                               nullptr);
         }
         __syncthreads();
     }
@@ -729,8 +757,8 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) wfa_walk_kernel(WalkArgs A) {
 constexpr size_t ALIGN = 256;
 inline size_t up(size_t x) { return (x + ALIGN - 1) & ~(ALIGN - 1); }
 
-// Threads of a forward block: wide ones while every wavefront fits a block's
-// shared memory.
+// Threads of a forward block: wide ones while every wavefront of a long pair
+// fits a block's shared memory.
 int forward_threads(int eff) { return eff <= block_scores(WFA_WIDE) ? WFA_WIDE : WFA_NARROW; }
 
 // Persistent grid: one wide block (two heavy pairs never share an SM while
@@ -741,38 +769,53 @@ int grid_blocks(int n_pairs, int eff) {
     return std::max(1, std::min(n_pairs, forward_threads(eff) == WFA_WIDE ? 148 : 296));
 }
 
-// Workspace pieces: [counters | spill slots | history]
+// Workspace pieces: [counters | last chunks | block slots | warp slots | history]
 struct Ws {
     unsigned* work;
     unsigned long long* hist_used;
+    unsigned* warp_slots;
     long long* hist_off;
-    int* spill;
+    int* block_spill;
+    short* warp_spill;
     int* hist;
     long long hist_cap;
 };
 
+// Longest distance of a pair that one warp computes (with its distance known
+// it is below WFA_LONG_D, and never leaves shared memory).
+int warp_eff(int eff) { return std::min(eff, WFA_LONG_LEN - 1); }
+
+// The pieces in order; returns the bytes before the history.
+size_t place(char* p, int n_pairs, int eff, int blocks, Ws& w) {
+    const size_t n = (size_t)(n_pairs > 0 ? n_pairs : 1);
+    const int threads = forward_threads(eff), we = warp_eff(eff);
+    const size_t warps = std::min(n, (size_t)blocks * (threads / 32));
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        char* q = p && bytes ? p + at : nullptr;
+        at += up(bytes);
+        return q;
+    };
+    w.work = (unsigned*)take(64);
+    w.hist_used = (unsigned long long*)(w.work + 2);
+    w.warp_slots = w.work + 6;
+    w.hist_off = (long long*)take(sizeof(long long) * n);
+    w.block_spill = (int*)take(eff > block_scores(threads) ? sizeof(int) * 2 * (2 * (size_t)eff + 5) * blocks : 0);
+    w.warp_spill = (short*)take(we > WFA_SMEM_S ? sizeof(short) * 2 * (2 * (size_t)we + 5) * warps : 0);
+    w.hist = (int*)(p + at);
+    return at;
+}
+
 size_t fixed_bytes(int n_pairs, int eff, int blocks) {
-    size_t b = up(64) + up(sizeof(long long) * (size_t)(n_pairs > 0 ? n_pairs : 1));
-    if (eff > WFA_SMEM_S) b += up(sizeof(int) * 2 * (2 * (size_t)eff + 5) * (size_t)blocks * (forward_threads(eff) / 32));
-    return b;
+    Ws w;
+    return place(nullptr, n_pairs, eff, blocks, w);
 }
 
 int carve(void* ws, size_t bytes, int n_pairs, int eff, int blocks, Ws& w) {
     const size_t need = fixed_bytes(n_pairs, eff, blocks);
     if (!ws || bytes < need) return GMF_ERR_WORKSPACE;
-    char* p = (char*)ws;
-    w.work = (unsigned*)p;
-    w.hist_used = (unsigned long long*)(p + 8);
-    p += up(64);
-    w.hist_off = (long long*)p;
-    p += up(sizeof(long long) * (size_t)(n_pairs > 0 ? n_pairs : 1));
-    w.spill = nullptr;
-    if (eff > WFA_SMEM_S) {
-        w.spill = (int*)p;
-        p += up(sizeof(int) * 2 * (2 * (size_t)eff + 5) * (size_t)blocks * (forward_threads(eff) / 32));
-    }
-    w.hist = (int*)p;
-    w.hist_cap = (long long)((bytes - (size_t)(p - (char*)ws)) / sizeof(int));
+    place((char*)ws, n_pairs, eff, blocks, w);
+    w.hist_cap = (long long)((bytes - need) / sizeof(int));
     return GMF_OK;
 }
 
@@ -800,7 +843,10 @@ WfaArgs base_args(const gmf_wfa_pairs* pairs, int32_t max_distance, int eff, con
     a.T = make_seq(pairs->target, t_total);
     a.max_distance = max_distance;
     a.eff = eff;
-    a.spill = w.spill;
+    a.warp_eff = warp_eff(eff);
+    a.block_spill = w.block_spill;
+    a.warp_spill = w.warp_spill;
+    a.warp_slots = w.warp_slots;
     a.work = w.work;
     a.hist_used = w.hist_used;
     a.hist_off = w.hist_off;
