@@ -24,6 +24,31 @@ from .chaining import AnchorCSR
 from .device import bind, require_cuda, to_device
 
 
+# Workspace of one seeding pass.  It takes about 12 bytes a base, and 8 KB for
+# a read shorter than a tile: 1,000,000 reads of 150 bp took 8.3 GB and 21.5 ms
+# at once, 1.4 GB and 22.2 ms in ranges of this size (0.9 GB and 22.5 ms, 0.6 GB
+# and 24.2 ms in ranges of a half and a quarter of it).
+SEED_WORKSPACE = 1 << 30
+
+
+def workspace_ranges(read_off: np.ndarray, budget: int) -> list:
+    """Consecutive ranges [r0, r1) of reads whose seeding workspaces are at
+    most ``budget`` bytes each; a read above it forms a range of its own."""
+    off = np.asarray(read_off, np.int64)
+    f, n, out, r0 = _native.lib().gmf_seed_workspace_bytes, len(off) - 1, [], 0
+    while r0 < n:
+        lo, hi = r0 + 1, n  # the most reads that fit
+        while lo < hi:
+            mid = (lo + hi + 1) // 2
+            if f(mid - r0, int(off[mid] - off[r0])) <= budget:
+                lo = mid
+            else:
+                hi = mid - 1
+        out.append((r0, lo))
+        r0 = lo
+    return out or [(0, 0)]
+
+
 class DeviceMinimizerIndex:
     def __init__(self, ref_codes: np.ndarray, k: int = 15, w: int = 10, max_occ: int = 0, device=None):
         from .synth import MinimizerSketch
@@ -64,40 +89,63 @@ class DeviceMinimizerIndex:
         anchors), read_pos, ref_pos, length, strand, the anchor count and the
         largest read's anchor count."""
         s = stream or torch.cuda.current_stream(self.device)
-        sp = int(s.cuda_stream)
-        bind(self.device, sp)
-        idx = self.c()
-        vp = ctypes.c_void_p
+        bind(self.device, int(s.cuda_stream))
         # every allocation and torch op on the caller's stream: the library's
         # kernels run there, and a worker's stream is not ordered with the
         # thread's default stream
+        with torch.cuda.stream(s):
+            need = int(_native.lib().gmf_seed_workspace_bytes(n_reads, int(codes_d.numel())))
+            if need <= SEED_WORKSPACE:
+                return self._seed_tiles(codes_d, read_off_d, n_reads, both_strands, s, need)
+            # a batch whose workspace would be larger is seeded in ranges of reads
+            h_off = read_off_d[: n_reads + 1].cpu().numpy()
+            parts = []
+            for r0, r1 in workspace_ranges(h_off, SEED_WORKSPACE):
+                c0, c1 = int(h_off[r0]), int(h_off[r1])
+                at = min(c0, codes_d.numel() - 1)  # a range of empty reads still has an address
+                codes = codes_d[at: max(c1, at + 1)]
+                need = int(_native.lib().gmf_seed_workspace_bytes(r1 - r0, int(codes.numel())))
+                parts.append(self._seed_tiles(codes, read_off_d[r0: r1 + 1] - c0, r1 - r0, both_strands, s, need))
+            if len(parts) == 1:
+                return parts[0]
+            n = [p["n_anchors"] for p in parts]
+            out = dict(n_anchors=sum(n), max_read_anchors=max(p["max_read_anchors"] for p in parts))
+            base = np.cumsum([0] + n)
+            out["read_off"] = torch.cat([p.pop("read_off")[: None if k == len(n) - 1 else -1] + int(base[k])
+                                         for k, p in enumerate(parts)])
+            for name in ("read_pos", "ref_pos", "length", "strand"):
+                out[name] = torch.cat([p.pop(name)[:t] for p, t in zip(parts, n)])
+                if out["n_anchors"] == 0:
+                    out[name] = out[name].new_empty(1)
+        return out
+
+    def _seed_tiles(self, codes_d: torch.Tensor, read_off_d: torch.Tensor, n_reads: int, both_strands: bool,
+                    s: torch.cuda.Stream, need: int) -> dict:
+        """seed_device in one workspace of ``need`` bytes, on the current stream ``s``."""
+        sp, vp, lib = int(s.cuda_stream), ctypes.c_void_p, _native.lib()
+        idx = self.c()
         total_codes = int(codes_d.numel())
         pre = _native.GmfSeedPrefix(self.prefix_bits, self.prefix.data_ptr()) if self.prefix is not None else None
         both = 1 if both_strands else 0
-        lib = _native.lib()
-        with torch.cuda.stream(s):
-            need = int(lib.gmf_seed_workspace_bytes(n_reads, total_codes))
-            ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
-            off = torch.empty(3 * n_reads + 4, dtype=torch.int64, device=self.device)
-            aoff, roff, totals = off[: 2 * n_reads + 1], off[2 * n_reads + 1: 3 * n_reads + 2], off[3 * n_reads + 2:]
-            _native.check("gmf_seed_scan", lib.gmf_seed_scan(
-                ctypes.byref(idx), ctypes.byref(pre) if pre is not None else None, n_reads, vp(codes_d.data_ptr()),
-                vp(read_off_d.data_ptr()), total_codes, both, vp(aoff.data_ptr()), vp(roff.data_ptr()),
-                vp(totals.data_ptr()), vp(ws.data_ptr()), ws.numel(), vp(sp)))
-            # the total sizes the outputs; the largest read is checked against the chaining limit (one
-            # host round trip for both)
-            total, most = (int(x) for x in totals.cpu().tolist())
-            i32 = dict(dtype=torch.int32, device=self.device)
-            out = dict(read_pos=torch.empty(max(total, 1), **i32), ref_pos=torch.empty(max(total, 1), **i32),
-                       length=torch.empty(max(total, 1), **i32),
-                       strand=torch.empty(max(total, 1), dtype=torch.int8, device=self.device))
-            _native.check("gmf_seed_emit", lib.gmf_seed_emit(
-                ctypes.byref(idx), n_reads, vp(read_off_d.data_ptr()), total_codes, both, vp(aoff.data_ptr()),
-                vp(out["read_pos"].data_ptr()), vp(out["ref_pos"].data_ptr()), vp(out["length"].data_ptr()),
-                vp(out["strand"].data_ptr()), vp(ws.data_ptr()), ws.numel(), vp(sp)))
-            out["read_off"] = roff
-        out["n_anchors"] = total
-        out["max_read_anchors"] = most
+        ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
+        off = torch.empty(3 * n_reads + 4, dtype=torch.int64, device=self.device)
+        aoff, roff, totals = off[: 2 * n_reads + 1], off[2 * n_reads + 1: 3 * n_reads + 2], off[3 * n_reads + 2:]
+        _native.check("gmf_seed_scan", lib.gmf_seed_scan(
+            ctypes.byref(idx), ctypes.byref(pre) if pre is not None else None, n_reads, vp(codes_d.data_ptr()),
+            vp(read_off_d.data_ptr()), total_codes, both, vp(aoff.data_ptr()), vp(roff.data_ptr()),
+            vp(totals.data_ptr()), vp(ws.data_ptr()), ws.numel(), vp(sp)))
+        # the total sizes the outputs; the largest read is checked against the chaining limit (one
+        # host round trip for both)
+        total, most = (int(x) for x in totals.cpu().tolist())
+        i32 = dict(dtype=torch.int32, device=self.device)
+        out = dict(read_pos=torch.empty(max(total, 1), **i32), ref_pos=torch.empty(max(total, 1), **i32),
+                   length=torch.empty(max(total, 1), **i32),
+                   strand=torch.empty(max(total, 1), dtype=torch.int8, device=self.device))
+        _native.check("gmf_seed_emit", lib.gmf_seed_emit(
+            ctypes.byref(idx), n_reads, vp(read_off_d.data_ptr()), total_codes, both, vp(aoff.data_ptr()),
+            vp(out["read_pos"].data_ptr()), vp(out["ref_pos"].data_ptr()), vp(out["length"].data_ptr()),
+            vp(out["strand"].data_ptr()), vp(ws.data_ptr()), ws.numel(), vp(sp)))
+        out.update(read_off=roff, n_anchors=total, max_read_anchors=most)
         return out
 
     def seed(self, reads: Sequence[np.ndarray], both_strands: bool = True) -> AnchorCSR:
