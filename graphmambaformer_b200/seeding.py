@@ -31,6 +31,10 @@ from .device import bind, require_cuda, to_device
 SEED_WORKSPACE = 1 << 30
 
 
+# Keys of an index that the tile pass can hold (it keeps 32-bit key numbers).
+TILE_KEYS = 2 ** 31 - 1
+
+
 def workspace_ranges(read_off: np.ndarray, budget: int) -> list:
     """Consecutive ranges [r0, r1) of reads whose seeding workspaces are at
     most ``budget`` bytes each; a read above it forms a range of its own."""
@@ -66,7 +70,7 @@ class DeviceMinimizerIndex:
         self.bytes = int(self.keys.numel() * 8 + self.offsets.numel() * 8 + self.positions.numel() * 4)
         # about one key per bucket, so a lookup is one load of the table and one or two of keys
         self.prefix = None
-        if 0 < self.n_keys < 2 ** 31:
+        if 0 < self.n_keys <= TILE_KEYS:
             self.prefix_bits = min(2 * self.k, 24, max(1, self.n_keys.bit_length()))
             self.prefix = torch.empty((1 << self.prefix_bits) + 1, dtype=torch.int32, device=self.device)
             s = torch.cuda.current_stream(self.device)
@@ -94,6 +98,8 @@ class DeviceMinimizerIndex:
         # kernels run there, and a worker's stream is not ordered with the
         # thread's default stream
         with torch.cuda.stream(s):
+            if self.n_keys > TILE_KEYS:
+                return self._seed_reads(codes_d, read_off_d, n_reads, both_strands, s)
             need = int(_native.lib().gmf_seed_workspace_bytes(n_reads, int(codes_d.numel())))
             if need <= SEED_WORKSPACE:
                 return self._seed_tiles(codes_d, read_off_d, n_reads, both_strands, s, need)
@@ -146,6 +152,32 @@ class DeviceMinimizerIndex:
             vp(out["read_pos"].data_ptr()), vp(out["ref_pos"].data_ptr()), vp(out["length"].data_ptr()),
             vp(out["strand"].data_ptr()), vp(ws.data_ptr()), ws.numel(), vp(sp)))
         out.update(read_off=roff, n_anchors=total, max_read_anchors=most)
+        return out
+
+    def _seed_reads(self, codes_d: torch.Tensor, read_off_d: torch.Tensor, n_reads: int, both_strands: bool,
+                    s: torch.cuda.Stream) -> dict:
+        """seed_device by one block per read and orientation, for an index of
+        any size, on the current stream ``s``."""
+        sp, vp, lib = int(s.cuda_stream), ctypes.c_void_p, _native.lib()
+        idx, both = self.c(), 1 if both_strands else 0
+        counts = torch.empty(max(2 * n_reads, 1), dtype=torch.int64, device=self.device)
+        _native.check("gmf_seed_count", lib.gmf_seed_count(
+            ctypes.byref(idx), n_reads, vp(codes_d.data_ptr()), vp(read_off_d.data_ptr()), both,
+            vp(counts.data_ptr()), vp(sp)))
+        aoff = torch.zeros(2 * n_reads + 1, dtype=torch.int64, device=self.device)
+        if n_reads:
+            torch.cumsum(counts[: 2 * n_reads], 0, out=aoff[1:])
+        per_read = (counts[0: 2 * n_reads: 2] + counts[1: 2 * n_reads: 2]).max() if n_reads else counts[0] * 0
+        total, most = (int(x) for x in torch.stack([aoff[-1], per_read]).cpu().tolist())
+        i32 = dict(dtype=torch.int32, device=self.device)
+        out = dict(read_pos=torch.empty(max(total, 1), **i32), ref_pos=torch.empty(max(total, 1), **i32),
+                   length=torch.empty(max(total, 1), **i32),
+                   strand=torch.empty(max(total, 1), dtype=torch.int8, device=self.device))
+        _native.check("gmf_seed_fill", lib.gmf_seed_fill(
+            ctypes.byref(idx), n_reads, vp(codes_d.data_ptr()), vp(read_off_d.data_ptr()), both, vp(aoff.data_ptr()),
+            vp(out["read_pos"].data_ptr()), vp(out["ref_pos"].data_ptr()), vp(out["length"].data_ptr()),
+            vp(out["strand"].data_ptr()), vp(sp)))
+        out.update(read_off=aoff[::2].contiguous(), n_anchors=total, max_read_anchors=most)
         return out
 
     def seed(self, reads: Sequence[np.ndarray], both_strands: bool = True) -> AnchorCSR:

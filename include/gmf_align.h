@@ -238,7 +238,8 @@ size_t gmf_seed_workspace_bytes(int32_t n_reads, int64_t total_codes);
  * forward, then reverse complement; the reverse ones empty when both_strands
  * is 0), read_anchor_off[n_reads + 1] (may be NULL) those of the reads,
  * totals[0] their number and totals[1] the largest read's.  prefix may be
- * NULL. */
+ * NULL.  An index of 2^31 keys or more is GMF_ERR_LIMIT (gmf_seed_count and
+ * gmf_seed_fill take it). */
 int gmf_seed_scan(const gmf_minimizer_index* index, const gmf_seed_prefix* prefix, int32_t n_reads,
                   const int8_t* codes, const int64_t* read_off, int64_t total_codes, int32_t both_strands,
                   int64_t* anchor_off, int64_t* read_anchor_off, int64_t* totals, void* workspace,
