@@ -38,7 +38,7 @@ from typing import Optional, Sequence
 import numpy as np
 import torch
 
-from . import _native
+from . import _native, wfa
 from .chaining import LUTS, AnchorCSR, ChainingConfig, chain_params
 from .config import ExtensionConfig
 from .device import bind, pack_host, packed_layout, require_cuda
@@ -53,12 +53,19 @@ from .session import _Buffers
 CIGAR_WITH_RESULTS = 256 << 10
 
 
-def estimate_bytes(read_lens: np.ndarray, n_anchors: int, cfg: ExtensionConfig, max_chains: int) -> int:
+def estimate_bytes(read_lens: np.ndarray, n_anchors: int, cfg: ExtensionConfig, max_chains: int,
+                   wavefronts: bool = True) -> int:
     """Upper bound on a batch's device working memory: anchors with the
-    chaining workspace, and every possible chain's traceback bits."""
+    chaining workspace, and every possible chain's traceback bits or, if that
+    is more, its wavefronts (they use the same buffer, one after the other;
+    left out without ``wavefronts``)."""
     W = 2 * cfg.max_half_band + 1
-    cells = int(np.sum((np.asarray(read_lens, np.int64) + 2 * cfg.flank) * W)) * min(max_chains, 2)
-    return int(120 * n_anchors + cells // 2 + 64 * len(read_lens) + (1 << 20))
+    span = np.asarray(read_lens, np.int64) + 2 * cfg.flank
+    chains = min(max_chains, 2)
+    extension = int(np.sum(span * W)) * chains // 2
+    if wavefronts and cfg.algorithm == "wfa" and len(span):
+        extension = max(extension, wfa.direct_bytes(np.repeat(span, chains), cfg.wfa_max_distance))
+    return int(120 * n_anchors + extension + 64 * len(read_lens) + (1 << 20))
 
 
 class BatchAlignments:
@@ -350,7 +357,6 @@ class BatchAligner:
         bound go to banded SW one chain per call, as the reference re-enters
         extend_chains."""
         from .extension import wfa_extension_result
-        from .wfa import DeviceWfaPairs, align_device_pairs
 
         cfg = self.ecfg
         rlen = rl[cr]
@@ -359,9 +365,10 @@ class BatchAligner:
         wend = np.minimum(self.ref_len, wstart + np.maximum(1, rlen + net))
         wlen = np.maximum(wend - wstart, 0)
         qd, qo_d, td, to_d, *_ = self._gather("w", reads_d, roff, rl, cr, rc, wstart, wlen)
-        dp = DeviceWfaPairs(len(cr), qd, qo_d, td, to_d, rlen.astype(np.int32), wlen.astype(np.int32), self.device)
-        res = align_device_pairs(dp, cfg.wfa_max_distance, stream=self.stream,
-                                 workspace=lambda nb: self.buf.device_buf("wws", nb, torch.uint8))
+        dp = wfa.DeviceWfaPairs(len(cr), qd, qo_d, td, to_d, rlen.astype(np.int32), wlen.astype(np.int32), self.device)
+        # the pairs beyond the bound follow in the same workspace
+        res = wfa.align_device_pairs(dp, cfg.wfa_max_distance, stream=self.stream,
+                                     workspace=lambda nb: self.buf.device_buf("sws", nb, torch.uint8))
         exts = [None] * len(cr)
         far = np.nonzero(res.distance < 0)[0]
         for c in np.nonzero(res.distance >= 0)[0]:
@@ -429,7 +436,9 @@ class AlignServer:
             n_anchors = int(a.read_off[-1])
         nb = estimate_bytes(rl, n_anchors, self.ecfg, self.ccfg.max_chains)
         if nb > self.budget:
-            raise ValueError("request larger than the working-memory budget")
+            if estimate_bytes(rl, n_anchors, self.ecfg, self.ccfg.max_chains, wavefronts=False) > self.budget:
+                raise ValueError("request larger than the working-memory budget")
+            nb = self.budget  # only the room kept for its wavefronts is above it: it runs by itself
         with self.lock:
             rid = self._next
             self._next += 1

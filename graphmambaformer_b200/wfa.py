@@ -332,6 +332,15 @@ def direct_entries(qlen: np.ndarray, tlen: np.ndarray, max_distance: int) -> int
     return int((1024 * c * c + 2 * c).sum())
 
 
+def direct_bytes(lens: np.ndarray, max_distance: int) -> int:
+    """Workspace with which align_device_pairs starts on pairs whose longer
+    sides are ``lens``."""
+    top = int(np.max(lens, initial=0))
+    md = max(0, min(int(max_distance), top))
+    entries = min(HISTORY_BUDGET, direct_entries(lens, lens, md))
+    return int(_native.lib().gmf_wfa_workspace_bytes(len(lens), top, md, entries))
+
+
 def _align_device(dp, max_distance, stream, sp, traceback, history_budget, workspace) -> WfaResult:
     dev, n = dp.device, dp.n
     if not traceback:
