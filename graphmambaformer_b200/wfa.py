@@ -350,9 +350,13 @@ def _align_device(dp, max_distance, stream, sp, traceback, history_budget, works
     md = _check_bound(max_distance, dp.max_len)
     lib = _native.lib()
     order = to_device(np.argsort(-(dp.h_qlen.astype(np.int64) + dp.h_tlen), kind="stable").astype(np.int32), dev)
-    need = int(lib.gmf_wfa_workspace_bytes(n, dp.max_len, md,
-                                           min(int(history_budget), direct_entries(dp.h_qlen, dp.h_tlen, md))))
-    ws = _ws(workspace, dev, need)
+    entries = min(int(history_budget), direct_entries(dp.h_qlen, dp.h_tlen, md))
+    need = int(lib.gmf_wfa_workspace_bytes(n, dp.max_len, md, entries))
+    try:
+        ws = _ws(workspace, dev, need)
+    except torch.OutOfMemoryError:  # no room for the guess: the distances alone, then histories of exact sizes
+        need = int(lib.gmf_wfa_workspace_bytes(n, dp.max_len, md, 0))
+        ws = _ws(workspace, dev, need)
     cap = int(dp.h_qlen.astype(np.int64).sum() + dp.h_tlen.astype(np.int64).sum() + n)
     # one buffer for the fixed-size results: starts and the word count, then counts, lengths, distances, flags
     fixed = torch.empty(2 * n + 2 + 6 * n + 1, dtype=torch.int32, device=dev)
