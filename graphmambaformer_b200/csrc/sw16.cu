@@ -1259,42 +1259,54 @@ int sw16_smem_per_warp(int cls, int ring, int tring, int tabn) {
     return (32 / L) * (int)group_smem_bytes(ring, tring, tabn);
 }
 
+// A wide band's rings bound the warps an SM holds, and 4 warps a block can leave
+// room that 2 or 3 would use: at half bands of 2,044 to 2,110 a warp takes 34 KB,
+// so one block of 4 fits an SM, or three of 2.  The warps a block are the most
+// (up to `wpb`) that keep the most resident.  1,200 pairs of 900 bp, half bands
+// 2,044 / 2,080: 9,082 / 9,237 us with 4 warps a block, 6,882 / 7,001 us so.
 template <int L, bool TB, bool XD, int EM>
-static int launch_l(const SwArgs& a, int grid, int wpb, cudaStream_t stream) {
+static int launch_l(const SwArgs& a, int wpb, cudaStream_t stream) {
     const int cls = L == 8 ? CLS_I16_L8 : (L == 16 ? CLS_I16_L16 : CLS_I16_L32);
-    const size_t smem = (size_t)sw16_smem_per_warp(cls, a.ring, a.tring, a.tabn) * wpb;
+    const size_t per_warp = (size_t)sw16_smem_per_warp(cls, a.ring, a.tring, a.tabn);
     void (*k)(SwArgs) = sw16_kernel<L, TB, XD, EM>;
-    if (smem > 48 * 1024)
-        GMF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    {  // persistent grid: every resident block of every SM
-        int dev = 0, sms = 0, per_sm = 0;
-        GMF_CUDA_TRY(cudaGetDevice(&dev));
-        GMF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        GMF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * wpb, smem));
-        grid = sms * (per_sm > 0 ? per_sm : 1);
+    if (per_warp * wpb > 48 * 1024)
+        GMF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(per_warp * wpb)));
+    int dev = 0, sms = 0, per_sm = 0;  // persistent grid: every resident block of every SM
+    GMF_CUDA_TRY(cudaGetDevice(&dev));
+    GMF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    GMF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * wpb, per_warp * wpb));
+    if (per_warp > 14 * 1024) {  // (below, 16 warps fit whatever the block)
+        for (int w = wpb - 1; w >= 1; --w) {
+            int n = 0;
+            GMF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 32 * w, per_warp * w));
+            if (n * w > per_sm * wpb) {
+                per_sm = n;
+                wpb = w;
+            }
+        }
     }
-    k<<<grid, 32 * wpb, smem, stream>>>(a);
+    k<<<sms * (per_sm > 0 ? per_sm : 1), 32 * wpb, per_warp * wpb, stream>>>(a);
     return cuda_status(cudaGetLastError());
 }
 
 template <int L, bool TB, bool XD>
-static int launch_le(const SwArgs& a, int e_mode, int grid, int wpb, cudaStream_t s) {
-    if (e_mode == 0) return launch_l<L, TB, XD, 0>(a, grid, wpb, s);
-    if (e_mode == 1) return launch_l<L, TB, XD, 1>(a, grid, wpb, s);
-    return launch_l<L, TB, XD, 2>(a, grid, wpb, s);
+static int launch_le(const SwArgs& a, int e_mode, int wpb, cudaStream_t s) {
+    if (e_mode == 0) return launch_l<L, TB, XD, 0>(a, wpb, s);
+    if (e_mode == 1) return launch_l<L, TB, XD, 1>(a, wpb, s);
+    return launch_l<L, TB, XD, 2>(a, wpb, s);
 }
 
 template <int L>
-static int launch_lx(const SwArgs& a, bool tb, bool xd, int e_mode, int grid, int wpb, cudaStream_t s) {
-    if (tb) return xd ? launch_le<L, true, true>(a, e_mode, grid, wpb, s) : launch_le<L, true, false>(a, e_mode, grid, wpb, s);
-    return xd ? launch_le<L, false, true>(a, e_mode, grid, wpb, s) : launch_le<L, false, false>(a, e_mode, grid, wpb, s);
+static int launch_lx(const SwArgs& a, bool tb, bool xd, int e_mode, int wpb, cudaStream_t s) {
+    if (tb) return xd ? launch_le<L, true, true>(a, e_mode, wpb, s) : launch_le<L, true, false>(a, e_mode, wpb, s);
+    return xd ? launch_le<L, false, true>(a, e_mode, wpb, s) : launch_le<L, false, false>(a, e_mode, wpb, s);
 }
 
-int launch_sw16(const SwArgs& a, int cls, bool tb, bool xd, int e_mode, int grid, int wpb,
+int launch_sw16(const SwArgs& a, int cls, bool tb, bool xd, int e_mode, int wpb,
                 cudaStream_t stream) {
-    if (cls == CLS_I16_L8) return launch_lx<8>(a, tb, xd, e_mode, grid, wpb, stream);
-    if (cls == CLS_I16_L16) return launch_lx<16>(a, tb, xd, e_mode, grid, wpb, stream);
-    return launch_lx<32>(a, tb, xd, e_mode, grid, wpb, stream);
+    if (cls == CLS_I16_L8) return launch_lx<8>(a, tb, xd, e_mode, wpb, stream);
+    if (cls == CLS_I16_L16) return launch_lx<16>(a, tb, xd, e_mode, wpb, stream);
+    return launch_lx<32>(a, tb, xd, e_mode, wpb, stream);
 }
 
 }  // namespace gmf

@@ -579,10 +579,9 @@ extern "C" int gmf_banded_sw(const gmf_pairs* pairs, const gmf_sw_params* params
         const int wpb = warps_per_block((size_t)sw16_smem_per_warp(c, ac.ring, ac.tring, ac.tabn), di,
                                         tun.warps_per_block);
         if (wpb == 0) return GMF_ERR_LIMIT;
-        const int grid = di.sms * std::max(1, 16 / wpb);
         cudaStream_t s;
         GMF_TRY(next_stream(&s));
-        GMF_TRY(launch_sw16(ac, c, tb, xd, em, grid, wpb, s));
+        GMF_TRY(launch_sw16(ac, c, tb, xd, em, wpb, s));
     }
     SwArgs a32 = a;
     a32.ring = ring_entries(std::max(64, Wmax + 1) - 64);

@@ -489,8 +489,7 @@ constexpr int L8_WMAX = 1021, L16_WMAX = 2045;
 // Launch helpers implemented by the kernel translation units.
 int launch_sw32(const SwArgs& a, bool tb, bool xd, int e_mode, bool queued, int grid, int wpb,
                 cudaStream_t stream);
-int launch_sw16(const SwArgs& a, int cls, bool tb, bool xd, int e_mode, int grid, int wpb,
-                cudaStream_t stream);
+int launch_sw16(const SwArgs& a, int cls, bool tb, bool xd, int e_mode, int wpb, cudaStream_t stream);
 int sw32_smem_per_warp(int ring);
 int sw16_smem_per_warp(int cls, int ring, int tring, int tabn);
 int launch_sw16_coop(const SwArgs& a, int cls, bool tb, bool xd, int e_mode, cudaStream_t stream);

@@ -261,7 +261,7 @@ typedef struct {
     int32_t l16_max_w;          /* ... up to this 16 lanes (>= l8_max_w); wider take a warp */
     int32_t coop_min_strips[3]; /* 2-, 4-, 8-warp classes: fewest 64-row strips a pair needs
                                    to be shared by that many warps; 0 disables the class */
-    int32_t warps_per_block;    /* one-warp classes: warps per CTA, 1..4 */
+    int32_t warps_per_block;    /* one-warp classes: warps per CTA at most, 1..4 */
     int32_t side_streams;       /* 1: class kernels overlap on side streams; 0: caller's stream */
 } gmf_sw_tuning;
 
