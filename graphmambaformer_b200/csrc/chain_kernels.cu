@@ -648,6 +648,20 @@ __global__ void __launch_bounds__(128) chain_dp_bcast_kernel(DpArgs a) {
 // 15 kb HiFi read 675 -> 268 us, 5,000 of them 1,874 -> 925 us (window 50),
 // 1,000 reads of 50-100 kb 5,011 -> 1,048 us (window 200).
 //
+// Anchors of repeats, on several diagonals at once, have their predecessors
+// beyond the nearest, and the rest of the window one anchor at a time takes
+// ~1,500 cycles.  So where the bound fails often, the next block scores whole
+// windows instead (dp_whole_block): every lane folds its own anchor's
+// candidates of the blocks before in one pass, which no f of this block holds
+// up, and the block's own as each of its f is broadcast.  It costs ~200 cycles
+// an anchor (window 64), a little more than the nearest alone, and so takes
+// over at 12 failures in 32 anchors: with 4 a read of one chain with gaps was
+// up to 9% slower, with 12 none by more than 2%.  The first block, whose whole
+// window is the block itself, is done so as well.  Whole calls (sort, DP and
+// peel) on one B200, the broadcast form / the nearest alone / both: one read of
+// 2,500 anchors on five diagonals 585 / 966 / 466 us, random anchors 999 / 2,119
+// / 823, 9,157 / 16,075 / 5,249 with a window of 1,000; 2,000 reads of 1,500
+// anchors on five diagonals 999 / 1,286 / 830.
 __device__ __forceinline__ double int_to_double(int x) {  // exact: one add instead of a conversion
     return __hiloint2double(0x43300000, x ^ (int)0x80000000) - 4503601774854144.0;  // 2^52 + 2^31
 }
@@ -664,8 +678,80 @@ __device__ __forceinline__ double2 dp_pair(int dq, int dr, int wl, bool in, unsi
 }
 
 constexpr int NEAR = 4;
+constexpr double NEAR_SLACK = 0.015625;  // of the bound, for a candidate's two roundings: |f| < 2^14 anchors * 2^31
+constexpr int WHOLE_FROM = 12;       // of 32 anchors, see above
 constexpr int NEAR_MAX_GAP = 16384;  // every block reads the whole penalty table once for its minimum
 constexpr int NEAR_WARPS = 2;        // per block: small blocks spread the long segments over the SMs
+
+// What the next block needs to know of the anchors before it.
+struct Tail {
+    double f1, f2, f3, f4;  // f of the four before, nearest first
+    double older;           // largest f before those
+    int far;                // anchors of the last block to which an older predecessor may have mattered
+};
+
+// A block of G anchors per group with their whole windows (q, r, wl: the
+// lane's anchor; qr_at, f_at: bytes of the group's rings in shared memory).
+// Not inlined, so that it takes no registers from the nearest-first loop.
+template <int G>
+__device__ __noinline__ Tail dp_whole_block(int qr_at, int f_at, int rm, int base, int n, int lb, unsigned mg,
+                                            const double* __restrict__ lut, int q, int r, int wl, double min_pen,
+                                            double* f_out, int32_t* parent_out, Tail t) {
+    extern __shared__ double2 near_smem[];
+    const int2* s_qr = reinterpret_cast<const int2*>(reinterpret_cast<unsigned char*>(near_smem) + qr_at);
+    double* s_f = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(near_smem) + f_at);
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), mine = base + gl;
+    const double w = int_to_double(wl);
+    double bs = -INFINITY;
+    int bj = -1;
+    auto fold = [&](int j, const int2& c, double fj, bool in) {
+        const int dq = q - c.x, dr = r - c.y;
+        const int mn = dq < dr ? dq : dr;
+        const unsigned gap = (unsigned)(dr > dq ? dr - dq : dq - dr);
+        const double sc = __dsub_rn(__dadd_rn(fj, int_to_double(mn < wl ? mn : wl)), __ldg(&lut[gap < mg ? gap : mg]));
+        if (in && (unsigned)(dq - 1) < mg && (unsigned)(dr - 1) < mg && sc > bs) {
+            bs = sc;
+            bj = j;
+        }
+    };
+#pragma unroll 8
+    for (int j = base > lb ? base - lb : 0; j < base; ++j) fold(j, s_qr[j & rm], s_f[j & rm], j >= mine - lb);
+#pragma unroll 4
+    for (int u = 0; u < G; ++u) {
+        const double fu = __shfl_sync(FULL_MASK, bs > w ? bs : w, u, G);
+        fold(base + u, s_qr[(base + u) & rm], fu, gl > u && gl - u <= lb);
+    }
+    const double fi = bs > w ? bs : w;
+    s_f[mine & rm] = fi;
+    if (mine < n) {
+        f_out[mine] = fi;
+        parent_out[mine] = bs > w ? bj : -1;
+    }
+    // how often the nearest alone would not have done: the largest f before each anchor's nearest four, in the bound
+    double up_to = mine < n ? fi : -INFINITY;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+        const double v = __shfl_up_sync(FULL_MASK, up_to, o, G);
+        if (gl >= o && v > up_to) up_to = v;
+    }
+    double before = t.older;
+    if (base > 0) {
+        before = gl >= 1 ? fmax(before, t.f4) : before;
+        before = gl >= 2 ? fmax(before, t.f3) : before;
+        before = gl >= 3 ? fmax(before, t.f2) : before;
+        before = gl >= 4 ? fmax(before, t.f1) : before;
+    }
+    const double in_block = __shfl_up_sync(FULL_MASK, up_to, NEAR + 1, G);
+    if (gl > NEAR) before = fmax(before, in_block);
+    const unsigned m = __ballot_sync(FULL_MASK, mine < n && before + (w - min_pen + NEAR_SLACK) >= fi);
+    t.far = __popc(G == 32 ? m : (m >> (lane & ~(G - 1))) & ((1u << (G & 31)) - 1u));
+    t.older = __shfl_sync(FULL_MASK, fmax(before, up_to), G - 1 - NEAR, G);
+    t.f1 = __shfl_sync(FULL_MASK, fi, G - 1, G);
+    t.f2 = __shfl_sync(FULL_MASK, fi, G - 2, G);
+    t.f3 = __shfl_sync(FULL_MASK, fi, G - 3, G);
+    t.f4 = __shfl_sync(FULL_MASK, fi, G - 4, G);
+    return t;
+}
 
 __host__ __device__ inline size_t near_smem_bytes(int G, int ring) {  // per group
     return (size_t)G * (NEAR * 16 + 16 + 8) + (size_t)ring * 16;
@@ -684,7 +770,10 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) chain_dp_near_kernel(DpArgs a
     double2* s_w = s_pair + G * NEAR;                              // [G] (weight, weight - smallest penalty + slack)
     double* s_f = reinterpret_cast<double*>(s_w + G);              // ring of f
     int2* s_qr = reinterpret_cast<int2*>(s_f + R);                 // ring of (read_end, ref_end)
-    int* s_p = reinterpret_cast<int*>(s_qr + R);                   // [G] age of a predecessor beyond the nearest, else 0
+    const int ring_at = (int)(reinterpret_cast<unsigned char*>(s_f) - reinterpret_cast<unsigned char*>(near_smem));
+    const int qr_at = (int)(reinterpret_cast<unsigned char*>(s_qr) - reinterpret_cast<unsigned char*>(near_smem));
+    int* s_p = reinterpret_cast<int*>(s_qr + R);                   // [G] age of a predecessor beyond the nearest, else 0;
+                                                                   // [G] the number of anchors that looked for one
     const int lb = a.lookback > 1 ? a.lookback : 1;
     const unsigned mg = a.max_gap > 0 ? (unsigned)a.max_gap : 0u;
     const double* __restrict__ lut = a.lut;
@@ -714,6 +803,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) chain_dp_near_kernel(DpArgs a
         const int blocks = __reduce_max_sync(FULL_MASK, (n + G - 1) / G);
         double f1 = 0.0, f2 = 0.0, f3 = 0.0, f4 = 0.0;  // f of the four anchors before
         double older = -INFINITY;                       // largest f before those
+        bool whole = true;                              // the block's anchors score their whole window
         int q, r, wl;
         double unused;
         dp_load_slot<false>(a, st, r0, gl, n, q, r, unused, wl);
@@ -723,16 +813,30 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) chain_dp_near_kernel(DpArgs a
             __syncwarp();
             s_qr[mine & rm] = make_int2(q, r);
             s_p[gl] = 0;
+            if (gl == 0) s_p[G] = 0;
             __syncwarp();
+            if (whole) {  // uniform over the warp
+                Tail t{f1, f2, f3, f4, older, 0};
+                const int bq = q, br = r, bl = wl;
+                dp_load_slot<false>(a, st, r0, mine + G, n, q, r, unused, wl);  // the next block
+                t = dp_whole_block<G>(qr_at, ring_at, rm, base, n, lb, mg, lut, bq, br, bl, min_pen, a.f + st,
+                                      a.parent + st, t);
+                f1 = t.f1;
+                f2 = t.f2;
+                f3 = t.f3;
+                f4 = t.f4;
+                older = t.older;
+                whole = __any_sync(FULL_MASK, t.far >= WHOLE_FROM * G / 32);
+                continue;
+            }
 #pragma unroll
             for (int d = 1; d <= NEAR; ++d) {
                 const int2 c = s_qr[(mine - d) & rm];
                 s_pair[gl * NEAR + d - 1] = dp_pair(q - c.x, r - c.y, wl, d <= mine && d <= lb && mine < n, mg, lut);
             }
             {
-                // the slack covers the candidates' two roundings: |f| < 2^14 anchors * 2^31
                 const double w = int_to_double(wl);
-                s_w[gl] = make_double2(w, mine < n ? w - min_pen + 0.015625 : -INFINITY);
+                s_w[gl] = make_double2(w, mine < n ? w - min_pen + NEAR_SLACK : -INFINITY);
             }
             dp_load_slot<false>(a, st, r0, mine + G, n, q, r, unused, wl);  // the next block
             __syncwarp();
@@ -756,6 +860,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) chain_dp_near_kernel(DpArgs a
                     double best = c1 > z ? c1 : z;
                     if (!(older + wi.y < best)) {
                         // an older predecessor may score as much: the rest of the window, oldest first
+                        if (gl == 0) ++s_p[G];
                         const int u = u0 + v, i = base + u;
                         const int lim = lb < i ? lb : i;
                         const int2 me = s_qr[i & rm];
@@ -815,6 +920,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) chain_dp_near_kernel(DpArgs a
                 a.f[st + mine] = fi;
                 a.parent[st + mine] = age ? mine - age : -1;
             }
+            whole = __any_sync(FULL_MASK, s_p[G] >= WHOLE_FROM * G / 32);
         }
     }
 }
