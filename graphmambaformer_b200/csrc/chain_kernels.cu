@@ -119,6 +119,9 @@ struct SortArgs {
     int64_t cap;               // anchors the sorted outputs can hold (-1: caller-sized)
     int64_t key_cap;           // anchors the caller's workspace covers (reads beyond SORT_CAP need it)
     int* err;
+    const double* lut;         // with min_pen: the penalty table, for the DP's bound
+    int max_gap;
+    double* min_pen;           // its smallest entry, or null
 };
 
 // Radix sort of a read's anchors in shared memory: 16-bit indices by 8-bit
@@ -134,11 +137,17 @@ struct SortArgs {
 // index) pairs took 78 stages for 4,096 keys (199,000 warp instructions for a
 // 15 kb read's 2,700 anchors) and went through global memory beyond that.
 // Measured on one B200: one 15 kb read 89 -> 28 us, 5,000 of them 1,275
-// -> 338 us, 1,000 reads of 10,000 anchors 2,172 -> 296 us.
+// -> 338 us, 1,000 reads of 10,000 anchors 2,172 -> 296 us.  The digit passes
+// want 5 blocks an SM (48 registers; with 4, 5,000 reads take 10% longer).
 constexpr int SORT_CAP = 4096;      // anchors a 256-thread block sorts; larger reads take 1,024 threads
 constexpr int SORT_CAP_BIG = 16384;
 constexpr int SORT_ROWS = 16;       // rows of 32 a warp takes at most (both: 512 anchors a warp)
 static_assert(SORT_CAP_BIG >= GMF_MAX_READ_ANCHORS, "a read's anchors fit the large block");
+// Up to RANK_CAP anchors are placed by counting the smaller ones, a thread
+// each, which takes less than the digit passes (2,000 reads in a whole call, by
+// digits / by counting: of 90 anchors 125 / 96 us, of 200 133 / 126, of 250 145
+// / 148).
+constexpr int RANK_CAP = 224;
 
 template <int T>
 struct SortSmem {
@@ -231,6 +240,54 @@ __device__ __forceinline__ unsigned block_max(SortSmem<T>& S, unsigned v, unsign
 
 __device__ __forceinline__ unsigned bits_of(unsigned v) { return 32u - __clz(v); }
 
+__device__ __forceinline__ void sort_small_read(const SortArgs& a, int r, int n) {
+    extern __shared__ __align__(16) unsigned sort_smem[];
+    unsigned long long* key = reinterpret_cast<unsigned long long*>(sort_smem);
+    const int x = threadIdx.x;
+    const int64_t a0 = a.read_off[r];
+    unsigned long long mine = ~0ull;  // (strand group, ref_end, read_end)
+    int len = 0;
+    if (x < n) {
+        const int8_t s = a.strand[a0 + x];
+        len = a.length[a0 + x];
+        mine = (s == 1 ? 0ull : (s == -1 ? 1ull : 2ull)) << 62 |
+               (unsigned long long)((unsigned)(a.ref_pos[a0 + x] + len) & 0x7fffffffu) << 31 |
+               ((unsigned)(a.read_pos[a0 + x] + len) & 0x7fffffffu);
+        key[x] = mine;
+    }
+    const int n0 = __syncthreads_count(x < n && mine >> 62 == 0);
+    const int m = __syncthreads_count(x < n && mine >> 62 < 2);
+    if (x < n && mine >> 62 < 2) {
+        int rank = 0;
+#pragma unroll 8
+        for (int y = 0; y < n; ++y) rank += key[y] < mine || (key[y] == mine && y < x);
+        a.perm[a0 + rank] = x;
+        if (a.len_s) a.len_s[a0 + rank] = len;
+        a.ref_end_s[a0 + rank] = (int32_t)((mine >> 31) & 0x7fffffffu);
+        a.read_end_s[a0 + rank] = (int32_t)(mine & 0x7fffffffu);
+    }
+    if (x == 0) {
+        a.n_plus[r] = n0;
+        a.n_minus[r] = m - n0;
+    }
+}
+
+// The penalty table's smallest entry, by a block of 256 threads.
+__device__ __forceinline__ void smallest_penalty(const double* __restrict__ lut, int max_gap, double* out) {
+    __shared__ double s_min[8];
+    double m = INFINITY;
+#pragma unroll 8
+    for (int x = threadIdx.x; x <= max_gap; x += 256) m = fmin(m, __ldg(&lut[x]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_xor_sync(FULL_MASK, m, o));
+    if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int x = 1; x < 8; ++x) m = fmin(m, s_min[x]);
+        *out = m;
+    }
+}
+
 template <int T>
 __device__ void sort_read(const SortArgs& a, int r, int n, unsigned* key, unsigned short* ia, unsigned short* ib,
                           SortSmem<T>& S, int* cnt) {
@@ -242,6 +299,10 @@ __device__ void sort_read(const SortArgs& a, int r, int n, unsigned* key, unsign
     const int8_t* sd = a.strand + a0;
     auto group = [&](int x) { return sd[x] == 1 ? 0u : (sd[x] == -1 ? 1u : 2u); };
     auto read_end = [&](int x) { return (unsigned)(rp[x] + ln[x]) & 0x7fffffffu; };
+    if (T == 256 && n <= RANK_CAP) {
+        sort_small_read(a, r, n);
+        return;
+    }
     if (tid < 3) cnt[tid] = 0;
     __syncthreads();
     // extremes, strand counts, and whether the anchors come in (strand, read_end) order
@@ -326,10 +387,11 @@ __device__ __forceinline__ int sort_count(const SortArgs& a, int r, int* error) 
     return *error ? -1 : n;
 }
 
-__global__ void __launch_bounds__(256) chain_sort_kernel(SortArgs a) {
-    extern __shared__ unsigned sort_smem[];
+__global__ void __launch_bounds__(256, 5) chain_sort_kernel(SortArgs a) {
+    extern __shared__ __align__(16) unsigned sort_smem[];
     __shared__ int cnt[3];
     const int r = blockIdx.x;
+    if (r == 0 && a.min_pen) smallest_penalty(a.lut, a.max_gap, a.min_pen);  // not by every block of the DP
     int error;
     const int n = sort_count(a, r, &error);
     if (n < 0) {
@@ -349,7 +411,7 @@ __global__ void __launch_bounds__(256) chain_sort_kernel(SortArgs a) {
 // Reads of more than SORT_CAP anchors: a block looks through every gridDim-th
 // read and sorts the large ones.
 __global__ void __launch_bounds__(1024) chain_sort_big_kernel(SortArgs a) {
-    extern __shared__ unsigned sort_smem[];
+    extern __shared__ __align__(16) unsigned sort_smem[];
     __shared__ int cnt[3];
     __shared__ int n_found, found[1024];
     unsigned short* ia = reinterpret_cast<unsigned short*>(sort_smem + SORT_CAP_BIG);
@@ -393,6 +455,7 @@ struct DpArgs {
     double* f;
     int32_t* parent;
     int32_t ring;            // ring entries per warp (power of two > lookback)
+    const double* min_pen;   // near: the table's smallest penalty
     bool near;               // sorted by this call with lengths as weights: at most GMF_MAX_READ_ANCHORS a segment
     int64_t cap;             // reads mode: anchors f / parent hold (-1: caller-sized)
 };
@@ -680,7 +743,7 @@ __device__ __forceinline__ double2 dp_pair(int dq, int dr, int wl, bool in, unsi
 constexpr int NEAR = 4;
 constexpr double NEAR_SLACK = 0.015625;  // of the bound, for a candidate's two roundings: |f| < 2^14 anchors * 2^31
 constexpr int WHOLE_FROM = 12;       // of 32 anchors, see above
-constexpr int NEAR_MAX_GAP = 16384;  // every block reads the whole penalty table once for its minimum
+constexpr int NEAR_MAX_GAP = 16384;  // one block of the sort reads the whole penalty table for its minimum
 constexpr int NEAR_WARPS = 2;        // per block: small blocks spread the long segments over the SMs
 
 // What the next block needs to know of the anchors before it.
@@ -760,7 +823,6 @@ __host__ __device__ inline size_t near_smem_bytes(int G, int ring) {  // per gro
 template <int G>
 __global__ void __launch_bounds__(32 * NEAR_WARPS) chain_dp_near_kernel(DpArgs a) {
     extern __shared__ double2 near_smem[];
-    __shared__ double s_min[NEAR_WARPS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, gl = lane & (G - 1);
     constexpr int GPW = 32 / G, UNROLL = 8;
     const int R = a.ring, rm = R - 1;  // R is a multiple of G: a block's entries never wrap
@@ -777,15 +839,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) chain_dp_near_kernel(DpArgs a
     const int lb = a.lookback > 1 ? a.lookback : 1;
     const unsigned mg = a.max_gap > 0 ? (unsigned)a.max_gap : 0u;
     const double* __restrict__ lut = a.lut;
-    // smallest penalty a candidate can take
-    double min_pen = INFINITY;
-#pragma unroll 8
-    for (unsigned x = threadIdx.x; x <= mg; x += 32 * NEAR_WARPS) min_pen = fmin(min_pen, __ldg(&lut[x]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) min_pen = fmin(min_pen, __shfl_xor_sync(FULL_MASK, min_pen, o));
-    if (lane == 0) s_min[wib] = min_pen;
-    __syncthreads();
-    for (int x = 0; x < NEAR_WARPS; ++x) min_pen = fmin(min_pen, s_min[x]);
+    const double min_pen = *a.min_pen;  // smallest penalty a candidate can take
 
     const int n_reads = a.n_segments >> 1;
     const int n_groups = gridDim.x * NEAR_WARPS * GPW;
@@ -1648,8 +1702,12 @@ int peel_smem_elems() { return 2048; }
 size_t sort_smem_bytes(int elems) { return (size_t)elems * (sizeof(unsigned long long) + sizeof(int)); }
 
 int launch_sort(const gmf_anchor_batch* an, const gmf_sorted_anchors* so, int32_t* len_s, int64_t cap,
-                int64_t key_cap, int* err, cudaStream_t stream) {
+                int64_t key_cap, int* err, cudaStream_t stream, const double* lut = nullptr, int max_gap = 0,
+                double* min_pen = nullptr) {
     SortArgs s;
+    s.lut = lut;
+    s.max_gap = max_gap;
+    s.min_pen = min_pen;
     s.n_reads = an->n_reads;
     s.read_off = an->read_off;
     s.read_pos = an->read_pos;
@@ -1669,6 +1727,7 @@ int launch_sort(const gmf_anchor_batch* an, const gmf_sorted_anchors* so, int32_
     GMF_CUDA_TRY(cudaFuncSetAttribute(chain_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small));
     chain_sort_kernel<<<an->n_reads, 256, small, stream>>>(s);
     GMF_CUDA_TRY(cudaGetLastError());
+    if (cap >= 0 && cap <= SORT_CAP) return GMF_OK;  // no read has more
     GMF_CUDA_TRY(cudaFuncSetAttribute(chain_sort_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)big));
     chain_sort_big_kernel<<<std::min(an->n_reads, 148), 1024, big, stream>>>(s);
     return cuda_status(cudaGetLastError());
@@ -1874,8 +1933,10 @@ extern "C" int gmf_chain_batch(const gmf_anchor_batch* an, const gmf_chain_param
     }
     GMF_CUDA_TRY(cudaMemsetAsync(err, 0, 256, stream));
     int st;
+    const bool near = !sorted_in && cp->max_gap <= NEAR_MAX_GAP;
+    double* min_pen = near ? (double*)(err + 2) : nullptr;  // behind the error word
     if (!sorted_in) {
-        st = launch_sort(an, &so, mem_tmp, (int64_t)A, (int64_t)A, err, stream);
+        st = launch_sort(an, &so, mem_tmp, (int64_t)A, (int64_t)A, err, stream, pen_lut, cp->max_gap, min_pen);
         if (st) return st;
     }
     DpArgs d{};
@@ -1896,7 +1957,8 @@ extern "C" int gmf_chain_batch(const gmf_anchor_batch* an, const gmf_chain_param
     d.f = f;
     d.parent = parent;
     d.cap = (int64_t)A;
-    d.near = !sorted_in && cp->max_gap <= NEAR_MAX_GAP;
+    d.near = near;
+    d.min_pen = min_pen;
     st = launch_dp(d, 2 * an->n_reads, stream);
     if (st) return st;
 
@@ -1937,10 +1999,12 @@ extern "C" int gmf_chain_batch(const gmf_anchor_batch* an, const gmf_chain_param
                                       (int)one_smem_bytes(ONE_CAP)));
     chain_one_kernel<<<an->n_reads, 128, one_smem_bytes(ONE_CAP), stream>>>(k);
     GMF_CUDA_TRY(cudaGetLastError());
-    GMF_CUDA_TRY(cudaFuncSetAttribute(chain_one_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)one_smem_bytes(ONE_CAP_BIG)));
-    chain_one_big_kernel<<<std::min(an->n_reads, 148), 512, one_smem_bytes(ONE_CAP_BIG), stream>>>(k);
-    GMF_CUDA_TRY(cudaGetLastError());
+    if (A > (size_t)ONE_CAP) {  // a strand may have more
+        GMF_CUDA_TRY(cudaFuncSetAttribute(chain_one_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)one_smem_bytes(ONE_CAP_BIG)));
+        chain_one_big_kernel<<<std::min(an->n_reads, 148), 512, one_smem_bytes(ONE_CAP_BIG), stream>>>(k);
+        GMF_CUDA_TRY(cudaGetLastError());
+    }
     const size_t smem = sort_smem_bytes(k.smem_elems);
     GMF_CUDA_TRY(cudaFuncSetAttribute(chain_peel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
