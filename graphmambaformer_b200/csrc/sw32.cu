@@ -205,7 +205,11 @@ __device__ void sw32_pair(const SwArgs& a, int p, const Grp<32>& grp, int2* ring
 }
 
 // Plain form: warp w aligns pair order[w] (or w).  Queued form: warps pull
-// pairs of class CLS_I32 from the device work queue.
+// pairs of class CLS_I32 from the device work queue.  As in the 16x2 form, the
+// first pair of each warp is fixed, one warp of every block before a second
+// one, so that a short list spreads over the SMs: with the first pairs going
+// to whichever warps asked first, 64 pairs of 2 kb took 3,396 us beside the
+// other classes' kernels, 300 of 1 kb 2,378 us; so 1,684 and 885 us.
 template <bool TB, bool XD, int EM, bool QUEUED>
 __global__ void __launch_bounds__(128) sw32_kernel(SwArgs a) {
     extern __shared__ int2 sw32_ring[];
@@ -217,12 +221,12 @@ __global__ void __launch_bounds__(128) sw32_kernel(SwArgs a) {
     if (QUEUED) {
         const int count = a.queue[N_CLASSES + CLS_I32];
         const int32_t* list = a.lists + (size_t)CLS_I32 * a.n_pairs;
-        for (;;) {
-            int idx = 0;
-            if (lane == 0) idx = atomicAdd(&a.queue[CLS_I32], 1);
-            idx = __shfl_sync(FULL_MASK, idx, 0);
-            if (idx >= count) break;
+        const int wave = (int)blockIdx.x / a.sms;
+        int idx = ((wib + wpb - wave % wpb) % wpb) * (int)gridDim.x + (int)blockIdx.x;
+        while (idx < count) {
             sw32_pair<TB, XD, EM>(a, list[idx], grp, ring);
+            if (lane == 0) idx = atomicAdd(&a.queue[CLS_I32], 1) + (int)gridDim.x * wpb;
+            idx = __shfl_sync(FULL_MASK, idx, 0);
         }
     } else {
         for (int w = blockIdx.x * wpb + wib; w < a.n_pairs; w += gridDim.x * wpb) {
