@@ -444,9 +444,12 @@ __device__ __forceinline__ bool wfa_is_long(const WfaArgs& A, int p) {
 
 // Blocks pull positions of the caller's order.  A block takes one position
 // and, when its pair is long, computes it with all its warps; otherwise it
-// takes a position more for each of its other warps and its warps compute one
-// pair each (a long pair among those goes first, block-wide).  With a
-// longest-first order every long pair gets a block of its own.
+// takes positions for its other warps as well and its warps compute one pair
+// each (a long pair among those goes first, block-wide).  With a longest-first
+// order every long pair gets a block of its own.  It takes as many as there
+// are pairs per block, so that a small batch spreads over the SMs: 500 pairs of
+// 2 kb with nothing in common took 25.4 ms by 32 a block (on 16 SMs), 9.8
+// ms so, 500 of 3 kb with 13% differences 3,482 and 1,624 us.
 template <Mode MODE, int T>
 __global__ void __launch_bounds__(T, T == WFA_WIDE ? 1 : 2) wfa_forward_kernel(WfaArgs A) {
     constexpr int WARPS = T / 32;
@@ -455,7 +458,7 @@ __global__ void __launch_bounds__(T, T == WFA_WIDE ? 1 : 2) wfa_forward_kernel(W
     __shared__ long long s_scratch;
     const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
     if (lane == 0) s_slot[wib] = -1;
-    const unsigned n = (unsigned)A.n_pairs;
+    const unsigned n = (unsigned)A.n_pairs, take = min((unsigned)WARPS, (n + gridDim.x - 1) / gridDim.x);
     for (;;) {
         if (tid == 0) {
             const unsigned first = atomicAdd(A.work, 1u);
@@ -464,8 +467,8 @@ __global__ void __launch_bounds__(T, T == WFA_WIDE ? 1 : 2) wfa_forward_kernel(W
             if (first < n) {
                 const int p = A.order ? A.order[first] : (int)first;
                 if (!wfa_is_long<MODE>(A, p)) {
-                    const unsigned more = atomicAdd(A.work, (unsigned)(WARPS - 1));
-                    for (int e = 1; e < WARPS; ++e)
+                    const unsigned more = atomicAdd(A.work, take - 1);
+                    for (unsigned e = 1; e < take; ++e)
                         if (more + e - 1 < n) s_pos[e] = (int)(more + e - 1);
                 }
             }
