@@ -229,26 +229,29 @@ class WfaResult:
         return words_to_cigar(self.cigar_words[s: s + n])
 
 
-def _sub_batch(dp: DeviceWfaPairs, dist_d: torch.Tensor, h_dist: np.ndarray, idx: np.ndarray) -> tuple:
-    """The pairs `idx` of dp as their own device batch (codes copied on the
-    device; offsets from the host lengths)."""
-    qo = np.zeros(dp.n + 1, np.int64)
-    np.cumsum(dp.h_qlen, out=qo[1:])
-    to = np.zeros(dp.n + 1, np.int64)
-    np.cumsum(dp.h_tlen, out=to[1:])
-    ql, tl = dp.h_qlen[idx], dp.h_tlen[idx]
-    sqo = np.zeros(len(idx) + 1, np.int64)
-    np.cumsum(ql, out=sqo[1:])
-    sto = np.zeros(len(idx) + 1, np.int64)
-    np.cumsum(tl, out=sto[1:])
-    dev = dp.device
-    gq = torch.cat([dp.query[qo[p]: qo[p + 1]] for p in idx]) if sqo[-1] else torch.zeros(1, dtype=torch.int8,
-                                                                                         device=dev)
-    gt = torch.cat([dp.target[to[p]: to[p + 1]] for p in idx]) if sto[-1] else torch.zeros(1, dtype=torch.int8,
-                                                                                          device=dev)
-    sub = DeviceWfaPairs(len(idx), gq, to_device(sqo, dev), gt, to_device(sto, dev), ql, tl, dev)
-    d_sub = dist_d[torch.as_tensor(idx, dtype=torch.long, device=dev)].contiguous()
-    return sub, d_sub, h_dist[idx]
+def _sub_batch(dp: DeviceWfaPairs, dist_d: torch.Tensor, h_dist: np.ndarray, idx: np.ndarray, sp: int) -> tuple:
+    """The pairs `idx` of dp (ascending) as their own device batch: the codes
+    gathered on the device by one launch a side (slices joined by torch took
+    2 us of host time each: 3,000 pairs of 500 bases with nothing in common,
+    16.7 ms a call, 7.2 so)."""
+    if len(idx) == dp.n:
+        return dp, dist_d, h_dist
+    dev, lib, sides = dp.device, _native.lib(), []
+    bind(dev, sp)
+    for codes, lens in ((dp.query, dp.h_qlen), (dp.target, dp.h_tlen)):
+        off = np.zeros(dp.n + 1, np.int64)
+        np.cumsum(lens, out=off[1:])
+        sub = np.zeros(len(idx) + 1, np.int64)
+        np.cumsum(lens[idx], out=sub[1:])
+        cols = to_device(np.concatenate([off[idx], sub]), dev)
+        n_d = to_device(lens[idx].astype(np.int32), dev)
+        out = torch.empty(max(int(sub[-1]), 1), dtype=torch.int8, device=dev)
+        sub_d = cols[len(idx):]
+        _native.check("gmf_gather_segments", lib.gmf_gather_segments(
+            ptr(codes), int(off[-1]), len(idx), ptr(cols), ptr(n_d), None, ptr(out), ptr(sub_d), ctypes.c_void_p(sp)))
+        sides += [out, sub_d]
+    batch = DeviceWfaPairs(len(idx), *sides, dp.h_qlen[idx], dp.h_tlen[idx], dev)
+    return batch, dist_d[to_device(idx, dev)].contiguous(), h_dist[idx]
 
 
 def _run_align(sub: DeviceWfaPairs, d_sub: torch.Tensor, h_d: np.ndarray, sp: int, workspace=None) -> dict:
@@ -385,7 +388,7 @@ def _align_device(dp, max_distance, stream, sp, traceback, history_budget, works
         dist_d = to_device(h_dist, dev)
         for c0, c1 in history_chunks((h_dist[left].astype(np.int64) + 1) ** 2, history_budget):
             idx = left[c0:c1]
-            sub, d_sub, h_d = _sub_batch(dp, dist_d, h_dist, idx)
+            sub, d_sub, h_d = _sub_batch(dp, dist_d, h_dist, idx, sp)
             out = _run_align(sub, d_sub, h_d, sp, workspace)
             part = {k: v.to("cpu", non_blocking=True) for k, v in out.items() if k != "cigar"}
             stream.synchronize()
