@@ -136,9 +136,10 @@ struct SortArgs {
 // What bounds it is the latency of a pass's rows; a bitonic sort of (key,
 // index) pairs took 78 stages for 4,096 keys (199,000 warp instructions for a
 // 15 kb read's 2,700 anchors) and went through global memory beyond that.
-// Measured on one B200: one 15 kb read 89 -> 28 us, 5,000 of them 1,275
-// -> 338 us, 1,000 reads of 10,000 anchors 2,172 -> 296 us.  The digit passes
-// want 5 blocks an SM (48 registers; with 4, 5,000 reads take 10% longer).
+// Measured on one B200: one 15 kb read 89 -> 32 us (4 of them the table's
+// minimum), 5,000 of them 1,275 -> 341 us, 1,000 reads of 10,000 anchors 2,172
+// -> 299 us.  The digit passes want 5 blocks an SM (48 registers; with 4, 5,000
+// reads take 10% longer).
 constexpr int SORT_CAP = 4096;      // anchors a 256-thread block sorts; larger reads take 1,024 threads
 constexpr int SORT_CAP_BIG = 16384;
 constexpr int SORT_ROWS = 16;       // rows of 32 a warp takes at most (both: 512 anchors a warp)
@@ -376,7 +377,9 @@ __device__ void sort_read(const SortArgs& a, int r, int n, unsigned* key, unsign
 
 // Anchors of read r, or -1 (with the error noted) when the read cannot be
 // sorted: too many anchors for one read, or beyond what the workspace holds.
-// Such a read gets no sorted anchors (so no chains).
+// Such a read gets no sorted anchors (so no chains).  (gmf_chain_sort refuses
+// reads of more than SORT_CAP anchors that its workspace does not cover, which
+// once held their keys: a caller may count on the error.)
 __device__ __forceinline__ int sort_count(const SortArgs& a, int r, int* error) {
     const int64_t a0 = a.read_off[r];
     const int n = (int)(a.read_off[r + 1] - a0);
@@ -708,8 +711,8 @@ __global__ void __launch_bounds__(128) chain_dp_bcast_kernel(DpArgs a) {
 // cycles an anchor for a window of 50, 8 blocks of 32 for 200).  A pull form
 // with one candidate per lane and two warp reductions per anchor took 100
 // instructions and 380 cycles.  Measured on one B200, DP kernel alone: one
-// 15 kb HiFi read 675 -> 268 us, 5,000 of them 1,874 -> 925 us (window 50),
-// 1,000 reads of 50-100 kb 5,011 -> 1,048 us (window 200).
+// 15 kb HiFi read 675 -> 263 us, 5,000 of them 1,874 -> 825 us (window 50),
+// 1,000 reads of 50-100 kb 5,011 -> 1,029 us (window 200).
 //
 // Anchors of repeats, on several diagonals at once, have their predecessors
 // beyond the nearest, and the rest of the window one anchor at a time takes

@@ -9,8 +9,9 @@
 // the largest penalty), so the biased "-inf" N = Z - (2*pmax + 2) = 2*pmax is
 // still >= 0 and every value the recurrences form stays in [pmax, smax + Z]
 // with smax = match * (min(qlen, tlen) + 1).  The classifier sends a pair here
-// only when smax + Z + 2*pmax + 64 <= 65535, so all cells are exact unsigned
-// 16-bit integers and the local-alignment floor is a three-way max with Z.
+// only when smax + Z + match <= 32768 (fits_int16), so all cells are exact
+// unsigned 16-bit integers, every difference that a traceback flag tests stays
+// within 15 bits, and the local-alignment floor is a three-way max with Z.
 // The step uses the DPX __viaddmax_u16x2 / __viaddmin_u16x2 / __vimax3_u16x2,
 // byte permutes and logic on the ALU pipe, and puts its adds on the FMA pipe
 // (16x2 adds of constants, multiply-adds): the ALU pipe issues at half rate
@@ -338,9 +339,10 @@ struct CoopLinks {
 // chunk's values at hand.  Bounds of 95, 80 and 72 registers (20, 24 and 28
 // warps an SM instead of 16) ran the same pairs at 709, 656 and 551 GCUPS
 // (32 lanes) and a lone warp's steps 10, 31 and 35% slower, so the kernels ask
-// for 16 warps an SM.  Pairs of 16 lanes, short and alike, take 20: their last
-// wave counts for more (2,000 / 10,000 / 20,000 pairs of 150 bp: 76 / 170 / 299
-// us with 16 warps, 70 / 162 / 308 us with 20).
+// for 16 warps an SM.  Pairs of 16 lanes, short and alike, take 20, which by the
+// rounds that a batch makes is better or worse (us a call with 16 / 20 warps: of
+// 150 bp 2,000 pairs 70 / 72, 4,700 91 / 105, 10,000 168 / 165, 20,000 299 / 313,
+// 50,000 705 / 702; 20,000 of 250 bp 558 / 615, 3,000 of 1,000 bp 622 / 504).
 template <int L, int NW, bool TB, bool XD, int EM>
 __device__ __forceinline__ void sw16_rows(const SwArgs& a, const PairGeo& G, bool active, const Grp<L>& grp,
                                           const GroupSmem& sm, int w, int nstrips, int n_chunks, int last_chunk,
@@ -1260,8 +1262,8 @@ int sw16_smem_per_warp(int cls, int ring, int tring, int tabn) {
 }
 
 // A wide band's rings bound the warps an SM holds, and 4 warps a block can leave
-// room that 2 or 3 would use: at half bands of 2,044 to 2,110 a warp takes 34 KB,
-// so one block of 4 fits an SM, or three of 2.  The warps a block are the most
+// room that 2 or 3 would use: at half bands of 2,043 to 2,108 a warp takes 34 KB,
+// so one block of 4 fits an SM, or two of 3.  The warps a block are the most
 // (up to `wpb`) that keep the most resident.  1,200 pairs of 900 bp, half bands
 // 2,044 / 2,080: 9,082 / 9,237 us with 4 warps a block, 6,882 / 7,001 us so.
 template <int L, bool TB, bool XD, int EM>

@@ -522,7 +522,7 @@ extern "C" int gmf_banded_sw(const gmf_pairs* pairs, const gmf_sw_params* params
     // side stream of its own (or, untuned-off, to the caller's stream too),
     // longest classes first; classes that the widest band rules out are not
     // launched.  10,000 pairs of 150 bp: 180 us with every class on a side
-    // stream, several of them empty, and four memsets before them; so: 170 us.
+    // stream, several of them empty, and four memsets before them; so: 170 us (168 now).
     SideStreams* ss = nullptr;
     const bool fork = tun.side_streams != 0;
     if (fork) {

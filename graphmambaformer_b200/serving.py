@@ -7,7 +7,7 @@ the minimizer index resident on the device and, per batch of reads, runs the
 classical path (alignment/seeding.py L1056-1101 MinimizerIndex seeding, then
 alignment/chaining.py L620-745 and alignment/extension.py L469-641):
 
-  0. with an index: ``gmf_seed_count`` / ``gmf_seed_fill`` on the device;
+  0. with an index: ``gmf_seed_scan`` / ``gmf_seed_emit`` on the device;
   1. ``gmf_chain_batch``: strand split + sort, DP, chain peeling, select;
   2. the window and band of every kept chain (extension.py L489-509, on the
      host from the chain records), then ``gmf_gather_segments`` builds the

@@ -340,7 +340,10 @@ typedef struct {
 } gmf_sorted_anchors;
 
 /* workspace: >= 256 + 24 * n_anchors bytes (gmf_chain_workspace_bytes is
- * always enough); it holds the sort of reads too large for shared memory. */
+ * always enough).  Its first word receives the error bits of
+ * gmf_chain_noalloc_error_flags.  Every read is sorted in shared memory; a
+ * read of more than 4,096 anchors is left out (bit 2, no sorted anchors) where
+ * the workspace does not have 24 bytes for each anchor up to its last one. */
 int gmf_chain_sort(const gmf_anchor_batch* anchors, const gmf_sorted_anchors* sorted,
                    void* workspace, size_t workspace_bytes, gmf_stream_t stream);
 
@@ -419,8 +422,8 @@ int gmf_chain_batch_noalloc(const gmf_anchor_batch* anchors, const gmf_chain_par
 /* Error word of the last gmf_chain_batch_noalloc call on the stream's device,
  * copied into *flags (device or host memory) on `stream`; with host memory,
  * read it after the stream has synchronised.  Bits: 1 = a read had more than
- * GMF_MAX_READ_ANCHORS anchors, 2 = a read's sort did not fit the scratch,
- * 4 = a read's anchors lay beyond n_anchors; each such read got zero chains.
+ * GMF_MAX_READ_ANCHORS anchors, 2 = gmf_chain_sort alone: the workspace did not
+ * cover a read of more than 4,096 anchors, 4 = a read's anchors lay beyond n_anchors; each such read got zero chains.
  * 0 = every read was chained.  No counterpart in the reference (its chainer
  * raises on the host instead). */
 int gmf_chain_noalloc_error_flags(int32_t* flags, gmf_stream_t stream);
